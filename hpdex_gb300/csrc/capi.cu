@@ -69,6 +69,7 @@ constexpr int kRankThreads = 1024;
 constexpr int kPlainStreams = 128;  // concurrent streams of the plain form (the device runs at
                                     // most 128 kernels at once)
 constexpr int kMeanThreads = 256;
+constexpr int kMeanFixedThreads = 512;
 
 struct DeviceInfo {
     int device = -1;
@@ -561,11 +562,15 @@ struct UploadLaunch {  // one chunk, straight from the host arrays (see upload_c
     }
 };
 template <class V>
-struct MeanLaunch {
-    static int run(const MeanArgs* a, dim3 grid, size_t smem, cudaStream_t s) {
-        auto k = group_mean_kernel<V, kMeanThreads>;
-        CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<grid, kMeanThreads, smem, s>>>(*a);
+struct MeanLaunch {  // smem 0: accumulators in global memory
+    static int run(const MeanArgs* a, int grid, size_t smem, cudaStream_t s) {
+        if (smem == 0) {
+            group_mean_kernel<V, kMeanThreads><<<grid, kMeanThreads, 0, s>>>(*a);
+        } else {
+            auto k = group_mean_fixed_kernel<V, kMeanFixedThreads>;
+            CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            k<<<grid, kMeanFixedThreads, smem, s>>>(*a);
+        }
         CUDA_TRY(cudaGetLastError());
         return HPDEX_OK;
     }
@@ -1784,46 +1789,57 @@ int matrix_group_mean(const hpdex_matrix* m, const int32_t* group_id, int64_t n_
                       int32_t include_zeros, double* out) {
     const long long n_rows = m->n_rows, n_cols = m->n_cols;
     if (n_rows > 0 && !group_id) return fail(HPDEX_ERR_ARGUMENT, "group_id is NULL");
-    std::vector<long long> rows_per((size_t)n_groups, 0);
-    for (long long r = 0; r < n_rows; ++r) {
-        const int g = group_id[r];
-        if (g >= 0 && g < n_groups) ++rows_per[(size_t)g];
-    }
+    const size_t G = (size_t)n_groups;
+    // fixed-point sums in shared memory while three words of sums and two counts per group fit
+    const size_t need = G * 20;
+    const bool fixed = n_groups < 65535 && need <= m->dev.smem_optin - 1024 && m->max_col_nnz < (1ll << 31);
     DevBuf<int32_t> gid;
-    DevBuf<long long> grows;
+    DevBuf<uint16_t> gid16;
+    DevBuf<unsigned int> grows;
     DevBuf<double> dout;
     DevBuf<unsigned char> acc;
     TRY(gid.alloc(std::max<long long>(n_rows, 1)));
-    TRY(grows.alloc((size_t)n_groups));
-    TRY(dout.alloc((size_t)(n_cols * n_groups)));
-    if (n_rows) CUDA_TRY(cudaMemcpy(gid.p, group_id, sizeof(int32_t) * n_rows, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(grows.p, rows_per.data(), sizeof(long long) * n_groups, cudaMemcpyHostToDevice));
+    TRY(grows.alloc(G));
+    if (fixed) TRY(gid16.alloc(std::max<long long>(n_rows, 1)));
+    // a page-locked result buffer is written by the kernel itself
+    cudaPointerAttributes at{};
+    const bool direct = cudaPointerGetAttributes(&at, out) == cudaSuccess && at.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    if (!direct) TRY(dout.alloc((size_t)n_cols * G));
+    if (n_rows) CUDA_TRY(cudaMemcpyAsync(gid.p, group_id, sizeof(int32_t) * n_rows, cudaMemcpyHostToDevice, 0));
+    CUDA_TRY(cudaMemsetAsync(grows.p, 0, sizeof(unsigned int) * G, 0));
+    if (n_rows) {
+        const int rg = (int)std::min<long long>((n_rows + 511) / 512, (long long)m->dev.sms * 2);
+        if (G <= 12288)
+            group_rows_kernel<true><<<rg, 512, G * sizeof(unsigned int)>>>(gid.p, n_rows, (int32_t)n_groups, grows.p, gid16.p);
+        else
+            group_rows_kernel<false><<<rg, 512>>>(gid.p, n_rows, (int32_t)n_groups, grows.p, gid16.p);
+        CUDA_TRY(cudaGetLastError());
+    }
     MeanArgs a{};
     a.data = m->data.p;
     a.rows = m->rows.p;
     a.indptr = m->indptr.p;
+    a.col_kmin = m->col_kmin.p;
+    a.col_kmax = m->col_kmax.p;
+    a.col_flags = m->col_has_zero.p;
     a.n_rows = n_rows;
     a.n_cols = (int32_t)n_cols;
     a.G = (int32_t)n_groups;
     a.gid = gid.p;
+    a.gid16 = gid16.p;
     a.group_rows = grows.p;
     a.include_zeros = include_zeros;
-    a.out = dout.p;
-    const size_t need = (size_t)n_groups * 16;
-    const size_t budget = std::min(m->dev.smem_optin, m->dev.smem_per_sm / 2);
-    const int grid = (int)std::min<long long>(n_cols, (long long)m->dev.sms * 4);
-    size_t smem = 0;
-    if (need <= budget) {
-        a.acc_in_smem = 1;
-        smem = need;
-    } else {
-        a.acc_in_smem = 0;
-        TRY(acc.alloc((size_t)grid * need));
+    a.out = direct ? out : dout.p;
+    int grid = (int)n_cols;
+    if (!fixed) {
+        grid = (int)std::min<long long>(n_cols, (long long)m->dev.sms * 4);
+        TRY(acc.alloc((size_t)grid * 16 * G));
         a.acc_global = acc.p;
     }
-    TRY(dispatch_dtype<MeanLaunch>(m->dtype, &a, dim3(grid), smem, (cudaStream_t)0));
-    CUDA_TRY(cudaDeviceSynchronize());
-    CUDA_TRY(cudaMemcpy(out, dout.p, sizeof(double) * n_cols * n_groups, cudaMemcpyDeviceToHost));
+    TRY(dispatch_dtype<MeanLaunch>(m->dtype, &a, grid, fixed ? need : (size_t)0, (cudaStream_t)0));
+    CUDA_TRY(cudaStreamSynchronize(0));
+    if (!direct) CUDA_TRY(cudaMemcpy(out, dout.p, sizeof(double) * (size_t)n_cols * G, cudaMemcpyDeviceToHost));
     return HPDEX_OK;
 }
 }  // namespace
