@@ -1235,13 +1235,14 @@ int hpdex_bh_fdr(const double* p, int64_t n, double* fdr) {
     TRY(device_info(dev));
     const int nb = (int)((n + kSortTile - 1) / kSortTile);
     DevBuf<unsigned long long> k0, k1;
-    DevBuf<uint32_t> v0, v1, counts, bad;
+    DevBuf<uint32_t> v0, v1, counts, totals, bad;
     DevBuf<double> agg, carry, out;
     TRY(k0.alloc((size_t)n));
     TRY(k1.alloc((size_t)n));
     TRY(v0.alloc((size_t)n));
     TRY(v1.alloc((size_t)n));
     TRY(counts.alloc((size_t)256 * nb));
+    TRY(totals.alloc(256));
     TRY(bad.alloc(1));
     TRY(agg.alloc((size_t)nb));
     TRY(carry.alloc((size_t)nb));
@@ -1249,7 +1250,7 @@ int hpdex_bh_fdr(const double* p, int64_t n, double* fdr) {
     cudaStream_t s = 0;
     CUDA_TRY(cudaMemcpyAsync(k0.p, p, sizeof(double) * n, cudaMemcpyHostToDevice, s));
     CUDA_TRY(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), s));
-    canonical_zero_kernel<<<std::min(nb, dev.sms * 8), 256, 0, s>>>(k0.p, n);
+    CUDA_TRY(cudaFuncSetAttribute(radix_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortScatterSmem));
     unsigned long long* kin = k0.p;
     unsigned long long* kout = k1.p;
     uint32_t* vin = nullptr;
@@ -1257,16 +1258,17 @@ int hpdex_bh_fdr(const double* p, int64_t n, double* fdr) {
     for (int pass = 0; pass < 8; ++pass) {
         const int shift = 8 * pass;
         radix_count_kernel<<<nb, kSortThreads, 0, s>>>(kin, n, shift, counts.p, nb);
-        radix_scan_kernel<<<1, 1024, 0, s>>>(counts.p, (long long)256 * nb);
-        radix_scatter_kernel<<<nb, kSortThreads, 0, s>>>(kin, vin, kout, vout, n, shift, counts.p, nb);
+        radix_scan_kernel<<<256, kSortThreads, 0, s>>>(counts.p, nb, totals.p);
+        radix_scatter_kernel<<<nb, kSortThreads, kSortScatterSmem, s>>>(kin, vin, kout, vout, n, shift, counts.p, totals.p, nb);
         CUDA_TRY(cudaGetLastError());
         std::swap(kin, kout);
         vin = vout;
         vout = (vout == v1.p) ? v0.p : v1.p;
     }
-    bh_block_min_kernel<<<nb, kSortThreads, 0, s>>>(kin, n, agg.p, bad.p);
+    double* adj = reinterpret_cast<double*>(kout);  // the sort's other key buffer is free now
+    bh_block_min_kernel<<<nb, kSortThreads, 0, s>>>(kin, n, adj, agg.p, bad.p);
     bh_carry_kernel<<<1, 1024, 0, s>>>(agg.p, nb, carry.p);
-    bh_apply_kernel<<<nb, kSortThreads, 0, s>>>(kin, vin, n, carry.p, out.p);
+    bh_apply_kernel<<<nb, kSortThreads, 0, s>>>(adj, vin, n, carry.p, out.p);
     CUDA_TRY(cudaGetLastError());
     uint32_t bad_h = 0;
     CUDA_TRY(cudaMemcpyAsync(&bad_h, bad.p, sizeof bad_h, cudaMemcpyDeviceToHost, s));
