@@ -204,7 +204,7 @@ def bh_fdr(p):
     """Benjamini-Hochberg adjusted p-values on the device (scipy's false_discovery_control)."""
     import numpy as np
     p = np.ascontiguousarray(np.asarray(p, dtype=np.float64)).reshape(-1)
-    out = np.empty_like(p)
+    out = result_array(p.shape)
     check(lib().hpdex_bh_fdr(p.ctypes.data, p.size, out.ctypes.data))
     return out
 
@@ -215,8 +215,8 @@ def fold_change(means_gene_major, n_genes: int, n_groups: int, clip_value: float
     m = np.ascontiguousarray(np.asarray(means_gene_major, dtype=np.float64)).reshape(-1)
     if m.size != n_genes * n_groups:
         raise ValueError("means must hold n_genes * n_groups values")
-    fold = np.empty((max(n_groups - 1, 0), n_genes), np.float64)
-    log2fold = np.empty_like(fold)
+    fold = result_array((max(n_groups - 1, 0), n_genes))
+    log2fold = result_array(fold.shape)
     check(lib().hpdex_fold_change(m.ctypes.data, int(n_genes), int(n_groups), float(clip_value),
                                   fold.ctypes.data, log2fold.ctypes.data))
     return fold, log2fold
