@@ -1860,7 +1860,11 @@ int matrix_group_mean(const hpdex_matrix* m, const int32_t* group_id, int64_t n_
 // =======================================================================================
 namespace {
 
+// A chunk holds at least kChunkEntries entries (the host link takes about 30 us for them, a chunk's
+// eleven launches, memsets and events about 25 us of host time); at most kPipelineChunks chunks.
+// With 12 chunks for every matrix a 2,000 x 500 call (9e4 entries) took 486 us, as one chunk 196 us.
 constexpr int kPipelineChunks = 12;
+constexpr long long kChunkEntries = 1ll << 19;
 constexpr int kComputeStreams = 2;  // chunks alternate between this many compute streams
 
 // Row ids come as int64 (`indices`, narrowed on the device through staging buffers) or as
@@ -1904,12 +1908,12 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
         return HPDEX_OK;
     }
 
-    // equal chunks of about nnz / kPipelineChunks entries (whole columns), uploaded in
-    // descending order of their longest column: the compute left after the last copy is
-    // about the last chunk's longest gene
+    // equal chunks of whole columns, uploaded in descending order of their longest column: the
+    // compute left after the last copy is about the last chunk's longest gene
     std::vector<long long> cb{0};
-    for (int k = 1; k < kPipelineChunks; ++k) {
-        const long long target = nnz / kPipelineChunks * k;
+    const long long chunks = std::max<long long>(1, std::min<long long>(nnz / kChunkEntries, kPipelineChunks));
+    for (long long k = 1; k < chunks; ++k) {
+        const long long target = nnz / chunks * k;
         const long long c = std::lower_bound(indptr, indptr + C + 1, target) - indptr;
         if (c > cb.back() && c < C) cb.push_back(c);
     }
@@ -1952,7 +1956,7 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
     int prio_least = 0, prio_greatest = 0;
     CUDA_TRY(cudaDeviceGetStreamPriorityRange(&prio_least, &prio_greatest));
     CUDA_TRY(cudaStreamCreateWithPriority(&r.copy, cudaStreamNonBlocking, prio_greatest));
-    CUDA_TRY(cudaStreamCreateWithFlags(&r.comp2, cudaStreamNonBlocking));
+    if (K > 1) CUDA_TRY(cudaStreamCreateWithFlags(&r.comp2, cudaStreamNonBlocking));
     r.ev.assign((size_t)(2 * K + 3), nullptr);
     for (auto& e : r.ev) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     cudaStream_t sx = r.copy;
@@ -1981,16 +1985,25 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
     };
 
     // the host-side plan (group sizes, reference checks, layout, allocations) runs on a helper
-    // thread while the first chunk is uploaded
+    // thread while the first of several chunks is uploaded
     hpdex_plan* praw = nullptr;
     int plan_status = HPDEX_OK;
     std::string plan_error;
     const int dev_id = m->dev.device;
-    std::thread planner([&] {
-        cudaSetDevice(dev_id);
+    auto make_plan = [&] {
         plan_status = plan_create(m.get(), group_id, n_targets, opt, &praw, false);
         if (plan_status != HPDEX_OK) plan_error = hpdex_last_error();
-    });
+    };
+    struct Joined {  // joined on every exit
+        std::thread t;
+        void join() { if (t.joinable()) t.join(); }
+        ~Joined() { join(); }
+    } planner;
+    if (K > 1)
+        planner.t = std::thread([&] {
+            cudaSetDevice(dev_id);
+            make_plan();
+        });
     // column pointers, then the first chunk; the per-chunk gene order while they upload
     int first_copy = HPDEX_OK;
     if (cudaMemcpyAsync(m->indptr.p, indptr, sizeof(int64_t) * ((size_t)C + 1), cudaMemcpyHostToDevice, sx) != cudaSuccess)
@@ -2002,7 +2015,8 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
         std::iota(ob, oe, (int32_t)cb[k]);
         std::stable_sort(ob, oe, [&](int32_t x, int32_t y) { return m->col_nnz[(size_t)x] > m->col_nnz[(size_t)y]; });
     }
-    planner.join();
+    if (K > 1) planner.join();
+    else make_plan();
     std::unique_ptr<hpdex_plan> p(praw);
     if (plan_status != HPDEX_OK) return fail(plan_status, "%s", plan_error.c_str());
     // the p-value kernel of each chunk writes U1 and P (straight into the caller's arrays
@@ -2016,17 +2030,19 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
     // a scratch set of their own.
     cudaStream_t sc2 = r.comp2;
     RankLayout lay2;
-    TRY(rank_layout(m->dev, dtype, (int)p->G, m->max_col_nnz, &lay2, p->nbl, p->cnt_mode));
     DevBuf<unsigned char> dk2, dg2, ek2, eg2, acc2;
     DevBuf<uint32_t> cnt2;
-    TRY(dk2.alloc(lay2.dk_bytes()));
-    TRY(dg2.alloc(lay2.dg_bytes()));
-    if (lay2.need_slab_scratch) {
-        TRY(ek2.alloc(lay2.dk_bytes()));
-        TRY(eg2.alloc(lay2.dg_bytes()));
+    if (K > 1) {
+        TRY(rank_layout(m->dev, dtype, (int)p->G, m->max_col_nnz, &lay2, p->nbl, p->cnt_mode));
+        TRY(dk2.alloc(lay2.dk_bytes()));
+        TRY(dg2.alloc(lay2.dg_bytes()));
+        if (lay2.need_slab_scratch) {
+            TRY(ek2.alloc(lay2.dk_bytes()));
+            TRY(eg2.alloc(lay2.dg_bytes()));
+        }
+        if (!lay2.acc_in) TRY(acc2.alloc(lay2.acc_bytes((int)p->G)));
+        TRY(cnt2.alloc(lay2.cnt_words((int)p->G)));
     }
-    if (!lay2.acc_in) TRY(acc2.alloc(lay2.acc_bytes((int)p->G)));
-    TRY(cnt2.alloc(lay2.cnt_words((int)p->G)));
     const long long T = p->T;
     CUDA_TRY(cudaMemcpyAsync(p->order.p, order.data(), sizeof(int32_t) * C, cudaMemcpyHostToDevice, p->stream));
 
@@ -2065,7 +2081,7 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
         cudaStream_t s, s2;
         ~Drain() {
             cudaStreamSynchronize(s);
-            cudaStreamSynchronize(s2);
+            if (s2) cudaStreamSynchronize(s2);
         }
     } drain{sc, sc2};
 
@@ -2081,8 +2097,10 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
     }
     cudaEvent_t ev_fork = r.ev[(size_t)(2 * K)], ev_join = r.ev[(size_t)(2 * K + 1)];
     cudaEvent_t ev_touch = r.ev[(size_t)(2 * K + 2)];
-    CUDA_TRY(cudaEventRecord(ev_fork, sc));
-    CUDA_TRY(cudaStreamWaitEvent(sc2, ev_fork, 0));
+    if (K > 1) {
+        CUDA_TRY(cudaEventRecord(ev_fork, sc));
+        CUDA_TRY(cudaStreamWaitEvent(sc2, ev_fork, 0));
+    }
     for (int j = 0; j < K; ++j) {
         const int k = seq[(size_t)j];
         const long long c0 = cb[k], c1 = cb[k + 1];
@@ -2143,8 +2161,10 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
         }
         if (j + 1 < K) TRY(enqueue_copy(j + 1));
     }
-    CUDA_TRY(cudaEventRecord(ev_join, sc2));
-    CUDA_TRY(cudaStreamWaitEvent(sc, ev_join, 0));
+    if (K > 1) {
+        CUDA_TRY(cudaEventRecord(ev_join, sc2));
+        CUDA_TRY(cudaStreamWaitEvent(sc, ev_join, 0));
+    }
     CUDA_TRY(cudaStreamSynchronize(sc));
     TRY(check_device_errors(p.get()));
     if (!direct) TRY(hpdex_plan_download(p.get(), U1_out, P_out));
