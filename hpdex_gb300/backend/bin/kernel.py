@@ -121,7 +121,7 @@ def group_mean(data, indices, indptr, group_id, n_groups, include_zeros=True, th
     indptr = _as_index(indptr)
     group_id = np.ascontiguousarray(np.asarray(group_id), dtype=np.int32)
     R, C, nnz = group_id.size, indptr.size - 1, data.size
-    out = _lib.result_array((max(C, 0) * n_groups,))
+    out = _lib.fetched_array((max(C, 0) * n_groups,))
     if n_groups == 0 or C <= 0:
         return _readonly(out)
     st = _lib.lib().hpdex_group_mean(_DTYPES[data.dtype], data.ctypes.data, indices.ctypes.data,

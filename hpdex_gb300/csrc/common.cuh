@@ -101,12 +101,17 @@ struct Val<double> {
     static __device__ __forceinline__ bool finite(double x) {
         return ((uint64_t)__double_as_longlong(x) & 0x7ff0000000000000ull) != 0x7ff0000000000000ull;
     }
-    static __device__ __forceinline__ bool zero(double x) { return x == 0.0; }
-    static __device__ __forceinline__ bool neg(double x) { return x < 0.0; }
+    // (on the bits: a comparison of doubles takes the FP64 pipe, 2 lanes a cycle on an SM)
+    static __device__ __forceinline__ uint64_t bits(double x) { return (uint64_t)__double_as_longlong(x); }
+    static __device__ __forceinline__ bool zero(double x) { return (bits(x) << 1) == 0ull; }
+    static __device__ __forceinline__ bool neg(double x) {  // not NaN
+        return bits(x) > 0x8000000000000000ull && bits(x) <= 0xfff0000000000000ull;
+    }
     static __device__ __forceinline__ Key key(double x) { return key_of_f64(x); }
     static __device__ __forceinline__ double to_double(double x) { return x; }
     static __device__ __forceinline__ bool small_int(double x) {
-        return fabs(x) < 2147483648.0 && x == trunc(x);
+        const int e = (int)((bits(x) >> 52) & 0x7ffull) - 1023;  // 2^e <= |x| < 2^(e + 1)
+        return zero(x) || (e >= 0 && e < 31 && (bits(x) << (12 + e)) == 0ull);
     }
     static __device__ __forceinline__ double from_key(Key k) { return f64_of_key(k); }
 };

@@ -67,7 +67,8 @@ struct RankTask {
     const unsigned long long* col_kmax;  //   (kmin > kmax: none)
     const uint32_t* col_has_zero;        // per column: bit 0 stores an explicit finite zero,
                                          // bit 1 stores a finite value that is not an integer
-                                         // of magnitude below 2^31 (no histogram path)
+                                         // of magnitude below 2^31 (no histogram path), bit 2
+                                         // repeats its values (column_ties_kernel)
     int64_t n_rows;
     int32_t n_cols;
     int32_t G;                 // n_targets + 1 (at most the launch's layout G)
@@ -97,6 +98,8 @@ struct RankArgs {
     const int32_t* order;      // genes in processing order [n_order]
     const uint16_t* order_task;  // task of each entry of `order` (null: all task 0)
     int32_t n_order;
+    const int32_t* n_order_dev;  // non-null: read instead of n_order (genes that the stream
+                                 // kernel left, mwu_stream.cuh)
     int32_t* queue;            // work counter (batched form)
     int32_t single_gene;       // >= 0: plain form, this gene of task 0 only
     int32_t G;                 // layout G: the largest task G of the launch
@@ -803,12 +806,14 @@ struct BucketMap {
                                           : (uint32_t)(t * __uint_as_float((uint32_t)(23 - e0 + 127) << 23));
             return x < 0.0f ? 0x80000000u - u : 0x80000000u + u;
         } else if constexpr (std::is_same_v<V, double>) {
-            const double x = f64_of_key(key), t = fabs(x);
-            const unsigned long long bits = (unsigned long long)__double_as_longlong(t);
+            // (in integers, off the FP64 pipe: floor(t * 2^(52 - E0)) is the mantissa shifted)
+            const bool negative = !(key >> 63);
+            const unsigned long long bits = (negative ? ~key : key) & 0x7fffffffffffffffull;
             const unsigned long long b0 = (unsigned long long)(e0 + 1023) << 52;
-            const unsigned long long u = bits >= b0 ? bits - b0 + (1ull << 52)
-                : (unsigned long long)(t * __longlong_as_double((long long)(52 - e0 + 1023) << 52));
-            return x < 0.0 ? 0x8000000000000000ull - u : 0x8000000000000000ull + u;
+            const int ex = (int)(bits >> 52), sh = e0 + 1023 - (ex ? ex : 1);
+            const unsigned long long mant = (bits & 0xfffffffffffffull) | (ex ? 1ull << 52 : 0ull);
+            const unsigned long long u = bits >= b0 ? bits - b0 + (1ull << 52) : sh < 64 ? mant >> sh : 0ull;
+            return negative ? 0x8000000000000000ull - u : 0x8000000000000000ull + u;
         } else {
             return key;
         }
@@ -1023,40 +1028,44 @@ static __device__ __noinline__ unsigned long long hist_gene(
 // stored elements), B (target tie terms), the stored counts nz and negatives ng, and T_ref;
 // zero_handling none also writes the per-test sample sizes. Sample-size errors and duplicate
 // row ids go to the task's error words (lowest gene * G + group wins).
+__device__ __forceinline__ void finalize_target(const RankTask* tk, int c, int G, int zh, int g,
+                                                unsigned long long A, unsigned long long B,
+                                                const uint32_t* nz, const uint32_t* ng,
+                                                unsigned long long T_ref) {
+    const size_t idx = (size_t)(g - 1) * tk->n_cols + c;
+    const unsigned long long nz1 = nz[0], nz2 = nz[g];
+    unsigned long long n1, n2, u2x2, ties;
+    if (zh == ZH_NONE) {
+        n1 = nz1;
+        n2 = nz2;
+        if (n1 < 2) atomicMin(&tk->err[0], (unsigned long long)c * G);
+        else if (n2 < 2) atomicMin(&tk->err[0], (unsigned long long)c * G + g);
+        u2x2 = A;
+        ties = T_ref + B;
+        tk->n2[idx] = (uint32_t)nz2;
+        if (g == 1) tk->n1[c] = (uint32_t)nz1;
+    } else {
+        n1 = (unsigned long long)tk->group_rows[0];
+        n2 = (unsigned long long)tk->group_rows[g];
+        if (nz1 > n1) atomicMin(&tk->err[1], (unsigned long long)c * G);
+        if (nz2 > n2) atomicMin(&tk->err[1], (unsigned long long)c * G + g);
+        const unsigned long long z1 = n1 - nz1, z2 = n2 - nz2;
+        if (zh == ZH_MIN) u2x2 = A + 2ull * z1 * nz2 + z1 * z2;
+        else if (zh == ZH_MAX) u2x2 = A + z2 * (2ull * nz1 + z1);
+        else u2x2 = A + 2ull * z1 * (nz2 - ng[g]) + z2 * (2ull * ng[0] + z1);
+        const unsigned long long zz = z1 + z2;
+        ties = T_ref + B + zz * zz * zz - zz;
+    }
+    const long long u1x2 = (long long)(2ull * n1 * n2) - (long long)u2x2;
+    tk->U1[idx] = (double)u1x2 * 0.5;
+    tk->tie[idx] = tk->tie_correction ? (double)ties : 0.0;
+}
 template <int NT>
 __device__ __forceinline__ void finalize_gene(const RankTask* tk, int c, int G, int zh, const Acc& acc,
                                               const uint32_t* nz, const uint32_t* ng,
                                               unsigned long long T_ref) {
-    const unsigned long long nz1 = nz[0];
-    for (int g = 1 + (int)threadIdx.x; g < G; g += NT) {
-        const size_t idx = (size_t)(g - 1) * tk->n_cols + c;
-        const unsigned long long nz2 = nz[g];
-        unsigned long long n1, n2, u2x2, ties;
-        if (zh == ZH_NONE) {
-            n1 = nz1;
-            n2 = nz2;
-            if (n1 < 2) atomicMin(&tk->err[0], (unsigned long long)c * G);
-            else if (n2 < 2) atomicMin(&tk->err[0], (unsigned long long)c * G + g);
-            u2x2 = acc.A[g];
-            ties = T_ref + acc.B[g];
-            tk->n2[idx] = (uint32_t)nz2;
-            if (g == 1) tk->n1[c] = (uint32_t)nz1;
-        } else {
-            n1 = (unsigned long long)tk->group_rows[0];
-            n2 = (unsigned long long)tk->group_rows[g];
-            if (nz1 > n1) atomicMin(&tk->err[1], (unsigned long long)c * G);
-            if (nz2 > n2) atomicMin(&tk->err[1], (unsigned long long)c * G + g);
-            const unsigned long long z1 = n1 - nz1, z2 = n2 - nz2;
-            if (zh == ZH_MIN) u2x2 = acc.A[g] + 2ull * z1 * nz2 + z1 * z2;
-            else if (zh == ZH_MAX) u2x2 = acc.A[g] + z2 * (2ull * nz1 + z1);
-            else u2x2 = acc.A[g] + 2ull * z1 * (nz2 - ng[g]) + z2 * (2ull * ng[0] + z1);
-            const unsigned long long zz = z1 + z2;
-            ties = T_ref + acc.B[g] + zz * zz * zz - zz;
-        }
-        const long long u1x2 = (long long)(2ull * n1 * n2) - (long long)u2x2;
-        tk->U1[idx] = (double)u1x2 * 0.5;
-        tk->tie[idx] = tk->tie_correction ? (double)ties : 0.0;
-    }
+    for (int g = 1 + (int)threadIdx.x; g < G; g += NT)
+        finalize_target(tk, c, G, zh, g, acc.A[g], acc.B[g], nz, ng, T_ref);
 }
 
 // HIST: the variant with the histogram path (launched when some column of the launch's tasks
@@ -1152,7 +1161,7 @@ __global__ void __launch_bounds__(NT, 1) mwu_rank_kernel(const RankArgs a) {
             first = false;
         } else {
             const int gi = atomicAdd(a.queue, 1);
-            if (gi < a.n_order) {
+            if (gi < (a.n_order_dev ? *a.n_order_dev : a.n_order)) {
                 c = a.order[gi];
                 ti = a.order_task ? (int)a.order_task[gi] : 0;
             }

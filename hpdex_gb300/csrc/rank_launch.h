@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "mwu_rank.cuh"
+#include "mwu_stream.cuh"
 
 namespace hpdex {
 // Launches mwu_rank_kernel<V> for the dtype code `dtype` (HPDEX_* codes).
@@ -27,4 +28,8 @@ HPDEX_RANK_DECL(u64)
 HPDEX_RANK_DECL(f32)
 HPDEX_RANK_DECL(f64)
 #undef HPDEX_RANK_DECL
+// mwu_stream_kernel<V> for float data: threads per CTA, launch
+constexpr int kStreamThreads = 1024;
+cudaError_t stream_launch_f32(const StreamArgs& a, int grid, size_t smem, cudaStream_t s);
+cudaError_t stream_launch_f64(const StreamArgs& a, int grid, size_t smem, cudaStream_t s);
 }  // namespace hpdex

@@ -115,7 +115,7 @@ class ResidentMatrix:
         gid = np.ascontiguousarray(np.asarray(group_id), dtype=np.int32)
         if gid.size != self.n_rows:
             raise ValueError(f"group_id has {gid.size} entries, the matrix {self.n_rows} rows")
-        out = _lib.result_array((max(self.n_cols, 0) * max(int(n_groups), 0),))
+        out = _lib.fetched_array((max(self.n_cols, 0) * max(int(n_groups), 0),))
         _lib.check(_lib.lib().hpdex_matrix_group_mean(self._h, gid.ctypes.data, int(n_groups),
                                                       int(bool(include_zeros)), out.ctypes.data))
         return out
@@ -188,6 +188,11 @@ class Plan:
                 "bucket_bits": bits.value,
                 "ms": {f"{c}/2^{b}": round(float(t), 4) for (c, b), t in zip(names, ms)}}
 
+    def set_stream(self, mode: int) -> None:
+        """Diagnostic: float genes on the stream kernel: long ones whose values seldom repeat (-1,
+        the default), none (0) or all (1); results do not change."""
+        _lib.check(_lib.lib().hpdex_plan_set_stream(self._h, int(mode)))
+
     def set_drain_wait(self, on: bool) -> None:
         """Diagnostic: on makes a warp of the rank kernel wait a bounded number of polls for a
         large bucket another warp is still listing (off, the default, leaves it to the pass after
@@ -195,11 +200,9 @@ class Plan:
         _lib.check(_lib.lib().hpdex_plan_set_drain_wait(self._h, int(bool(on))))
 
     def download(self):
-        # page-locked buffers of the library's pool when it has them: fresh pageable pages fault one
-        # by one under the copy (the screen's 64 MB: 15 ms against 0.4 ms)
         C = self.matrix.n_cols
-        U1 = _lib.result_array((self.n_targets, C))
-        P = _lib.result_array((self.n_targets, C))
+        U1 = _lib.fetched_array((self.n_targets, C))
+        P = _lib.fetched_array((self.n_targets, C))
         _lib.check(_lib.lib().hpdex_plan_download(self._h, U1.ctypes.data, P.ctypes.data))
         return U1, P
 

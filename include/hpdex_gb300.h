@@ -245,6 +245,10 @@ int hpdex_plan_autotune(hpdex_plan* p, int32_t reps, int32_t* run_counters_out,
  * (the default) restores the per-gene choice. Both give the same results. */
 int hpdex_plan_set_histogram(hpdex_plan* p, int32_t on);
 
+/* Diagnostic: which genes of a batched run take the stream kernel (float matrices): -1 (default) long
+ * genes whose values seldom repeat, 0 none, 1 all. Results do not change. */
+int hpdex_plan_set_stream(hpdex_plan* plan, int32_t mode);
+
 /* Diagnostic. The rank kernel lets a warp resolve a large bucket while other warps of its CTA
  * are still listing them. By default (on = 0) a warp that finds the next list entry not yet
  * published leaves it to a pass after the next block barrier; on = 1 makes it wait for the entry
