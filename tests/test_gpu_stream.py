@@ -1,8 +1,9 @@
 """The stream kernel (all genes forced onto it, and the plan's own choice) against the rank kernel
-(the plain form runs it for every gene): U1 and P bit for bit, where the stream kernel can go wrong: pairs of equal
-(value, group) counted directly and through the bitmap with one or more partitions, genes it
-leaves (too many reference elements, crowded buckets), signed and wide ranges, heavy ties, empty and
-tiny genes, explicit zeros, non-finite values, row ids outside the matrix, few and many groups."""
+(the plain form runs it for every gene): U1 and P bit for bit, where the stream kernel can go
+wrong: pairs of equal (value, group) found through the bitmap and counted in one or more
+partitions, genes it leaves (too many reference elements, crowded buckets), signed and wide
+ranges, heavy ties, empty and tiny genes, explicit zeros, non-finite values, row ids outside the
+matrix, few and many groups."""
 import numpy as np
 import pytest
 
@@ -68,9 +69,13 @@ def _check(kind, dtype, n_rows, sizes, ref, T, in_group=1.0, bad_rows=False, **o
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("kind", ["log", "normal", "few", "one", "crowded", "wide", "dirty"])
 def test_stream_equals_rank(kind, dtype, zero):
-    """Genes from empty to 20,000 entries: direct tables, then the bitmap."""
-    _check(kind, dtype, 20_000, [0, 1, 2, 31, 33, 127, 129, 1_000, 4_097, 9_000, 13_001, 20_000], 2_500,
-           23, zero_handling=zero, use_continuity=True, bad_rows=kind == "dirty")
+    """Genes from empty to 20,000 entries (fewer where the rank kernel, which gives the expected
+    values, compares a gene's elements pairwise)."""
+    sizes = [0, 1, 2, 31, 33, 127, 129, 1_000, 4_097, 9_000, 13_001, 20_000]
+    if kind in ("crowded", "wide"):
+        sizes = [0, 1, 33, 600, 4_097]
+    _check(kind, dtype, 20_000, sizes, 2_500, 23, zero_handling=zero, use_continuity=True,
+           bad_rows=kind == "dirty")
 
 
 @pytest.mark.parametrize("kind,T,ref", [("log", 1, 4_000), ("log", 501, 12_000), ("normal", 60, 9_000),
