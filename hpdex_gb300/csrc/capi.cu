@@ -423,7 +423,8 @@ struct hpdex_plan {
     DevBuf<long long> d_group_rows;
     DevBuf<PConst> d_pconst;  // per-target p-value constants (zero_handling min / max / mix)
     DevBuf<int32_t> order;
-    DevBuf<int32_t> queue;       // work counters: rank kernel, stream kernel, genes left
+    DevBuf<int32_t> queue;       // work counters: rank kernel, stream kernel, genes left, histogram
+                                 // kernel
     DevBuf<int32_t> queue_init;  // their values before a batched run with the stream kernel
     DevBuf<int32_t> order_stream;  // the stream kernel's genes (n_stream; 0: not used)
     DevBuf<int32_t> left;        // the rank kernel's genes then: its own, and those the stream
@@ -443,6 +444,8 @@ struct hpdex_plan {
     DevBuf<uint32_t> cnt;
     RankArgs ra{};
     StreamArgs sa{};             // stream kernel of the batched form (use_stream)
+    HistArgs ha{};               // histogram kernel of the batched form (use_hist)
+    size_t hist_smem = 0;        // 0: the layout leaves no room for it
     size_t stream_smem = 0;      // 0: the layout leaves no room for it
     bool hist_on = true;         // histogram path allowed (hpdex_plan_set_histogram)
     int nbl = 13;                // bucket table of 2^nbl entries (hpdex_plan_set_bucket_bits)
@@ -829,6 +832,21 @@ size_t stream_layout(const DeviceInfo& dev, int dtype, int G, const RankLayout& 
     return fixed + (size_t)a->region;
 }
 
+// The histogram kernel's shared memory: kHistCTAs to an SM, fewer where 64 values of every group
+// need more, down to one; 0 when not even 8 values of every group fit (or the group ids are 32-bit).
+size_t hist_layout(const DeviceInfo& dev, int G, const RankLayout& r, HistArgs* a) {
+    if (!r.acc_in) return 0;
+    for (int ctas = kHistCTAs; ctas >= 1; --ctas) {
+        const size_t room = std::min(dev.smem_per_sm / ctas - dev.smem_reserved, dev.smem_optin) - 2048;
+        const size_t acc = hist_acc_bytes(G), values = ctas > 1 ? 64 : 8;
+        if (room < acc + 4 * (4 + values * (size_t)G)) continue;
+        a->G = G;
+        a->words = (int32_t)((room - acc) / 16 * 4);
+        return acc + 4 * (size_t)a->words;
+    }
+    return 0;
+}
+
 int configure_rank(hpdex_plan* p) {
     const hpdex_matrix* m = p->m;
     const int G = (int)p->G;
@@ -861,6 +879,17 @@ int configure_rank(hpdex_plan* p) {
     a.any_compact = t.compact_decode;
     set_layout_args(a, r, G, p->dk.p, p->dg.p, p->ek.p, p->eg.p, p->acc.p, p->cnt.p);
 
+    p->hist_smem = m->has_int_cols ? hist_layout(m->dev, G, r, &p->ha) : 0;
+    if (p->hist_smem) {
+        TRY(p->left.alloc(std::max<long long>(m->n_cols, 1)));
+        HistArgs& h = p->ha;
+        h.tasks = p->d_task.p;
+        h.order = p->order.p;
+        h.n_order = (int32_t)m->n_cols;
+        h.queue = p->queue.p + 3;
+        h.n_left = p->queue.p + 2;
+        h.left = p->left.p;
+    }
     p->stream_smem = p->n_stream ? stream_layout(m->dev, m->dtype, G, r, &p->sa) : 0;
     if (p->stream_smem) {
         StreamArgs& sa = p->sa;
@@ -902,10 +931,10 @@ int stream_genes(hpdex_plan* p, const std::vector<int32_t>& order) {
         if (stream) entries += m->col_nnz[(size_t)c];
     }
     if (entries * 2 < m->nnz || mine.empty()) return HPDEX_OK;
-    const int32_t init[3] = {0, 0, (int32_t)rest.size()};
+    const int32_t init[4] = {0, 0, (int32_t)rest.size(), 0};
     TRY(p->order_stream.alloc(mine.size()));
     TRY(p->left.alloc(order.size()));
-    TRY(p->queue_init.alloc(3));
+    TRY(p->queue_init.alloc(4));
     CUDA_TRY(cudaMemcpy(p->order_stream.p, mine.data(), sizeof(int32_t) * mine.size(), cudaMemcpyHostToDevice));
     if (!rest.empty()) CUDA_TRY(cudaMemcpy(p->left.p, rest.data(), sizeof(int32_t) * rest.size(), cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(p->queue_init.p, init, sizeof init, cudaMemcpyHostToDevice));
@@ -913,7 +942,9 @@ int stream_genes(hpdex_plan* p, const std::vector<int32_t>& order) {
     return HPDEX_OK;
 }
 
-// The stream kernel is off while a matrix holds integer columns (histogram path).
+// The stream kernel is off while a matrix holds integer columns (histogram path); the histogram
+// kernel takes those.
+bool use_hist(const hpdex_plan* p) { return p->hist_smem != 0 && !p->ra.no_histogram; }
 bool use_stream(const hpdex_plan* p) { return p->stream_smem != 0 && p->ra.no_histogram; }
 
 int launch_pvalues_asymptotic(hpdex_plan* p, cudaStream_t s) {
@@ -1130,10 +1161,18 @@ int enqueue_rank(hpdex_plan* p, int mode, cudaStream_t s, int* launches) {
     if (mode == HPDEX_MODE_BATCHED) {
         p->ra.single_gene = -1;
         RankArgs a = p->ra;
-        if (!use_stream(p)) {
+        if (use_hist(p)) {
+            CUDA_TRY(cudaMemsetAsync(p->queue.p, 0, 4 * sizeof(int32_t), s));
+            HistArgs h = p->ha;
+            h.erfc_table = a.erfc_table;
+            TRY(rank_status(hist_launch(p->m->dtype, h, p->m->dev.sms, p->hist_smem, s), "histogram kernel launch"));
+            *launches += 1;
+            a.order = p->left.p;
+            a.n_order_dev = h.n_left;
+        } else if (!use_stream(p)) {
             CUDA_TRY(cudaMemsetAsync(p->queue.p, 0, sizeof(int32_t), s));
         } else {  // the rank kernel then takes its own genes and those the stream kernel left
-            CUDA_TRY(cudaMemcpyAsync(p->queue.p, p->queue_init.p, 3 * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
+            CUDA_TRY(cudaMemcpyAsync(p->queue.p, p->queue_init.p, 4 * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
             StreamArgs sa = p->sa;
             sa.erfc_table = a.erfc_table;
             auto launch = p->m->dtype == HPDEX_FLOAT32 ? stream_launch_f32 : stream_launch_f64;
@@ -1549,7 +1588,7 @@ int plan_create(hpdex_matrix* m, const int32_t* group_id, int64_t n_targets,
         CUDA_TRY(cudaMemcpy(p->order.p, order.data(), sizeof(int32_t) * C, cudaMemcpyHostToDevice));
         TRY(stream_genes(p.get(), order));
     }
-    TRY(p->queue.alloc(3));
+    TRY(p->queue.alloc(4));
     TRY(p->err.alloc(kErrWords));
     const size_t n = (size_t)(p->T * C);
     TRY(p->U1.alloc(std::max<size_t>(n, 1)));
@@ -1607,7 +1646,7 @@ int hpdex_plan_run(hpdex_plan* p, int32_t mode) {
             CUDA_TRY(cudaGraphInstantiate(&p->graph_exec, g, 0));
         }
         CUDA_TRY(cudaGraphLaunch(p->graph_exec, s));
-        launches = (p->m->n_cols > 0 ? (use_stream(p) ? 3 : 2) : 0) + (!p->fused_pvalues && p->T * p->m->n_cols > 0 ? 1 : 0);
+        launches = (p->m->n_cols > 0 ? (use_stream(p) || use_hist(p) ? 3 : 2) : 0) + (!p->fused_pvalues && p->T * p->m->n_cols > 0 ? 1 : 0);
     } else {
         CUDA_TRY(cudaEventRecord(p->ev[0], s));
         CUDA_TRY(cudaMemsetAsync(p->err.p, 0xff, kErrWords * sizeof(unsigned long long), s));

@@ -20,6 +20,19 @@ cudaError_t HPDEX_CAT(rank_launch_, HPDEX_RANK_T)(const RankArgs& a, int grid, s
     return cudaGetLastError();
 }
 
+cudaError_t HPDEX_CAT(hist_launch_, HPDEX_RANK_T)(const HistArgs& a, int sms, size_t smem,
+                                                  cudaStream_t s) {
+    auto k = mwu_hist_kernel<HPDEX_RANK_V, kHistThreads, kHistCTAs>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    int blocks = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, kHistThreads, smem);
+    if (e != cudaSuccess) return e;
+    const int grid = blocks * sms < a.n_order ? blocks * sms : a.n_order;
+    k<<<grid, kHistThreads, smem, s>>>(a);
+    return cudaGetLastError();
+}
+
 cudaError_t HPDEX_CAT(rank_occupancy_, HPDEX_RANK_T)(size_t smem, size_t smem_optin,
                                                      int acc_in_smem, int* blocks) {
     // the variants of an accumulator layout get the same shared-memory limit

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "mwu_hist.cuh"
 #include "mwu_rank.cuh"
 #include "mwu_stream.cuh"
 
@@ -13,10 +14,13 @@ cudaError_t rank_launch(int dtype, const RankArgs& a, int grid, size_t smem, cud
 // many CTAs of `smem` bytes fit on an SM.
 cudaError_t rank_occupancy(int dtype, size_t smem, size_t smem_optin, int acc_in_smem,
                            int* blocks);
+// Launches mwu_hist_kernel<V> with as many CTAs of `smem` bytes as fit on `sms` SMs.
+cudaError_t hist_launch(int dtype, const HistArgs& a, int sms, size_t smem, cudaStream_t s);
 // per-type implementations
 #define HPDEX_RANK_DECL(T)                                                                    \
     cudaError_t rank_launch_##T(const RankArgs& a, int grid, size_t smem, cudaStream_t s);   \
-    cudaError_t rank_occupancy_##T(size_t smem, size_t smem_optin, int acc_in_smem, int* blocks);
+    cudaError_t rank_occupancy_##T(size_t smem, size_t smem_optin, int acc_in_smem, int* blocks); \
+    cudaError_t hist_launch_##T(const HistArgs& a, int sms, size_t smem, cudaStream_t s);
 HPDEX_RANK_DECL(i8)
 HPDEX_RANK_DECL(u8)
 HPDEX_RANK_DECL(i16)
