@@ -408,7 +408,9 @@ struct hpdex_matrix {
     DevBuf<uint32_t> col_has_zero;
     std::vector<long long> col_nnz;  // host copy for scheduling
     long long max_col_nnz = 0;
-    std::vector<uint8_t> col_ties;  // resident float matrices: the column's values repeat (else empty)
+    // resident float matrices whose long columns seldom repeat their values: which columns take the
+    // stream kernel (else empty)
+    std::vector<uint8_t> col_stream;
     bool has_int_cols = true;  // some column stores only small integers (launches then use the
                                // rank kernel with the histogram path)
     DeviceInfo dev;
@@ -588,6 +590,14 @@ struct MeanLaunch {  // smem 0: accumulators in global memory
     }
 };
 
+// Which genes take the stream kernel: those of at least kStreamMinEntries entries whose values
+// seldom repeat (a gene of 1,024 entries: 1.13 of the rank kernel's speed there, 20 groups; of 500:
+// 0.98, 100 groups), in a matrix where they hold kStreamMinPercent of the entries: the two kernels
+// run one after the other, each with a tail of its own (half the genes of a 100,000 x 2,000 log
+// matrix on each: 200 + 410 us, all on the rank kernel 430).
+constexpr long long kStreamMinEntries = 1024;
+constexpr long long kStreamMinPercent = 95;
+
 // Sets m->has_int_cols from the column flags of the key-range pass: some column with finite
 // nonzero values, all of them small integers (bit 1 of col_has_zero clear).
 // For float data first which columns repeat their values (column_ties_kernel).
@@ -610,9 +620,16 @@ int matrix_int_hint(hpdex_matrix* m) {
     CUDA_TRY(cudaMemcpy(hi.data(), m->col_kmax.p, sizeof(unsigned long long) * C, cudaMemcpyDeviceToHost));
     for (long long c = 0; c < C && !m->has_int_cols; ++c)
         m->has_int_cols = !(f[(size_t)c] & 2u) && lo[(size_t)c] <= hi[(size_t)c];
-    if (floats) {
-        m->col_ties.resize((size_t)C);
-        for (long long c = 0; c < C; ++c) m->col_ties[(size_t)c] = (f[(size_t)c] >> 2) & 1u;
+    if (floats && !m->has_int_cols) {
+        m->col_stream.resize((size_t)C);
+        long long mine = 0, all = 0;
+        for (long long c = 0; c < C; ++c) {
+            const long long n = m->col_nnz[(size_t)c];
+            m->col_stream[(size_t)c] = n >= kStreamMinEntries && !(f[(size_t)c] & 4u);
+            all += n;
+            if (m->col_stream[(size_t)c]) mine += n;
+        }
+        if (mine == 0 || mine * 100 < all * kStreamMinPercent) m->col_stream.clear();
     }
     return HPDEX_OK;
 }
@@ -681,14 +698,13 @@ int upload_matrix(hpdex_matrix* m, const void* data, const int64_t* indices, con
                                            (cudaStream_t)0));
         CUDA_TRY(cudaDeviceSynchronize());
     }
-    TRY(matrix_int_hint(m));
     m->col_nnz.resize((size_t)m->n_cols);
     m->max_col_nnz = 0;
     for (long long c = 0; c < m->n_cols; ++c) {
         m->col_nnz[(size_t)c] = indptr[c + 1] - indptr[c];
         m->max_col_nnz = std::max(m->max_col_nnz, m->col_nnz[(size_t)c]);
     }
-    return HPDEX_OK;
+    return matrix_int_hint(m);
 }
 
 // Whether a grouping leaves enough rows out (more than 15 %) for the rank kernel to keep only
@@ -894,7 +910,7 @@ int configure_rank(hpdex_plan* p) {
     if (p->stream_smem) {
         StreamArgs& sa = p->sa;
         sa.tasks = p->d_task.p;
-        sa.order = p->order_stream.p;
+        sa.order = p->order_stream.p ? p->order_stream.p : p->order.p;
         sa.n_order = p->n_stream;
         sa.queue = p->queue.p + 1;
         sa.n_left = p->queue.p + 2;
@@ -906,11 +922,7 @@ int configure_rank(hpdex_plan* p) {
     return HPDEX_OK;
 }
 
-// Divides a plan's genes (`order`, longest first) between the stream kernel, which takes the long
-// genes of a float matrix whose values seldom repeat, and the rank kernel. The two run one after
-// the other, so the stream kernel is used only when it takes most of the entries. A gene of
-// 1,024 entries: 1.13 of the rank kernel's time there (20 groups), of 500: 0.98 (100 groups).
-constexpr long long kStreamMinEntries = 1024;
+// Divides a plan's genes (`order`, longest first) between the stream kernel and the rank kernel.
 std::vector<int32_t> longest_first(const hpdex_matrix* m) {
     std::vector<int32_t> order((size_t)m->n_cols);
     std::iota(order.begin(), order.end(), 0);
@@ -922,22 +934,20 @@ std::vector<int32_t> longest_first(const hpdex_matrix* m) {
 int stream_genes(hpdex_plan* p, const std::vector<int32_t>& order) {
     const hpdex_matrix* m = p->m;
     p->n_stream = 0;
-    if (m->col_ties.empty() || m->has_int_cols || p->stream_mode == 0) return HPDEX_OK;
+    if (p->stream_mode == 0 || (p->stream_mode < 0 && m->col_stream.empty())) return HPDEX_OK;
     std::vector<int32_t> mine, rest;
-    long long entries = 0;
-    for (const int32_t c : order) {
-        const bool stream = p->stream_mode == 1 || (!m->col_ties[(size_t)c] && m->col_nnz[(size_t)c] >= kStreamMinEntries);
-        (stream ? mine : rest).push_back(c);
-        if (stream) entries += m->col_nnz[(size_t)c];
-    }
-    if (entries * 2 < m->nnz || mine.empty()) return HPDEX_OK;
+    for (const int32_t c : order)
+        (p->stream_mode == 1 || m->col_stream[(size_t)c] ? mine : rest).push_back(c);
+    if (mine.empty()) return HPDEX_OK;
     const int32_t init[4] = {0, 0, (int32_t)rest.size(), 0};
-    TRY(p->order_stream.alloc(mine.size()));
     TRY(p->left.alloc(order.size()));
-    TRY(p->queue_init.alloc(4));
-    CUDA_TRY(cudaMemcpy(p->order_stream.p, mine.data(), sizeof(int32_t) * mine.size(), cudaMemcpyHostToDevice));
-    if (!rest.empty()) CUDA_TRY(cudaMemcpy(p->left.p, rest.data(), sizeof(int32_t) * rest.size(), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(p->queue_init.p, init, sizeof init, cudaMemcpyHostToDevice));
+    TRY(p->order_stream.alloc(rest.empty() ? 0 : mine.size()));  // (all genes: p->order)
+    TRY(p->queue_init.alloc(rest.empty() ? 0 : 4));
+    if (!rest.empty()) {
+        CUDA_TRY(cudaMemcpy(p->order_stream.p, mine.data(), sizeof(int32_t) * mine.size(), cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpy(p->left.p, rest.data(), sizeof(int32_t) * rest.size(), cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpy(p->queue_init.p, init, sizeof init, cudaMemcpyHostToDevice));
+    }
     p->n_stream = (int)mine.size();
     return HPDEX_OK;
 }
@@ -1172,7 +1182,10 @@ int enqueue_rank(hpdex_plan* p, int mode, cudaStream_t s, int* launches) {
         } else if (!use_stream(p)) {
             CUDA_TRY(cudaMemsetAsync(p->queue.p, 0, sizeof(int32_t), s));
         } else {  // the rank kernel then takes its own genes and those the stream kernel left
-            CUDA_TRY(cudaMemcpyAsync(p->queue.p, p->queue_init.p, 4 * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
+            if (p->queue_init.p)
+                CUDA_TRY(cudaMemcpyAsync(p->queue.p, p->queue_init.p, 4 * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
+            else
+                CUDA_TRY(cudaMemsetAsync(p->queue.p, 0, 4 * sizeof(int32_t), s));
             StreamArgs sa = p->sa;
             sa.erfc_table = a.erfc_table;
             auto launch = p->m->dtype == HPDEX_FLOAT32 ? stream_launch_f32 : stream_launch_f64;
@@ -2376,6 +2389,8 @@ struct ServerQuery {
 struct ServerBatch {
     std::vector<ServerQuery*> q;
     DevBuf<RankTask> tasks;
+    // items (gene, query) of the histogram, stream and rank kernels, in this order; the rank
+    // kernel's part has room for what the others leave
     DevBuf<int32_t> order, queue;
     DevBuf<uint16_t> order_task;
     DevBuf<unsigned char> dk, dg, ek, eg, acc;
@@ -2506,29 +2521,47 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
         t.err = q->err.p;
         t.compact_decode = compact_decode(q->group_rows, R);
     }
-    // one work queue over every (query, gene) item of the batch, longest first by nnz class
-    std::vector<int32_t> order;
-    std::vector<uint16_t> order_task;
-    order.reserve((size_t)items);
-    order_task.reserve((size_t)items);
+    // a work queue per kernel over the (query, gene) items of the batch, longest first by nnz class:
+    // integer matrices to the histogram kernel, long float genes whose values seldom repeat to the
+    // stream kernel, the others to the rank kernel
+    HistArgs ha{};
+    StreamArgs sa{};
+    const size_t hist_smem = hist_layout(S->dev, GL, r, &ha);
+    const size_t stream_smem = stream_layout(S->dev, dtype, GL, r, &sa);
+    std::vector<int32_t> order[3];
+    std::vector<uint16_t> order_task[3];
+    auto put = [&](int list, int32_t c, size_t i) {
+        order[list].push_back(c);
+        order_task[list].push_back((uint16_t)i);
+    };
     for (int k = 63; k >= 0; --k)
         for (size_t i = 0; i < b.q.size(); ++i) {
+            const hpdex_matrix* m = S->mats[(size_t)b.q[i]->matrix];
             const auto& ord = S->mat_order[(size_t)b.q[i]->matrix];
             const auto& seg = S->mat_class_start[(size_t)b.q[i]->matrix];
             const int64_t lo = seg[(size_t)(2 * k)], hi = seg[(size_t)(2 * k + 1)];
-            order.insert(order.end(), ord.begin() + lo, ord.begin() + hi);
-            order_task.insert(order_task.end(), (size_t)(hi - lo), (uint16_t)i);
+            const bool hist = hist_smem && m->has_int_cols;
+            for (int64_t j = lo; j < hi; ++j) {
+                const int32_t c = ord[(size_t)j];
+                put(hist ? 0 : stream_smem && !m->col_stream.empty() && m->col_stream[(size_t)c] ? 1 : 2, c, i);
+            }
         }
+    const size_t n_hist = order[0].size(), n_stream = order[1].size(), n_rank = order[2].size();
+    const size_t n_items = n_hist + n_stream + n_rank, left_at = n_hist + n_stream, places = left_at + n_items;
     TRY(b.tasks.alloc(tasks.size()));
-    TRY(b.order.alloc(std::max<size_t>(order.size(), 1)));
-    TRY(b.order_task.alloc(std::max<size_t>(order.size(), 1)));
-    TRY(b.queue.alloc(1));
+    TRY(b.order.alloc(std::max<size_t>(places, 1)));
+    TRY(b.order_task.alloc(std::max<size_t>(places, 1)));
+    TRY(b.queue.alloc(4));
     CUDA_TRY(cudaMemcpyAsync(b.tasks.p, tasks.data(), sizeof(RankTask) * tasks.size(), cudaMemcpyHostToDevice, st));
-    if (!order.empty()) {
-        CUDA_TRY(cudaMemcpyAsync(b.order.p, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaMemcpyAsync(b.order_task.p, order_task.data(), sizeof(uint16_t) * order.size(), cudaMemcpyHostToDevice, st));
+    size_t at = 0;
+    for (int l = 0; l < 3; ++l) {
+        if (order[l].empty()) continue;
+        CUDA_TRY(cudaMemcpyAsync(b.order.p + at, order[l].data(), sizeof(int32_t) * order[l].size(), cudaMemcpyHostToDevice, st));
+        CUDA_TRY(cudaMemcpyAsync(b.order_task.p + at, order_task[l].data(), sizeof(uint16_t) * order[l].size(), cudaMemcpyHostToDevice, st));
+        at += order[l].size();
     }
-    CUDA_TRY(cudaMemsetAsync(b.queue.p, 0, sizeof(int32_t), st));
+    const int32_t counters[4] = {0, 0, (int32_t)n_rank, 0};  // rank, stream, left, histogram
+    CUDA_TRY(cudaMemcpyAsync(b.queue.p, counters, sizeof counters, cudaMemcpyHostToDevice, st));
 
     // results go straight into the caller's arrays when they are page-locked (result buffers
     // of hpdex_host_buffer_acquire) or when the device reaches pageable memory; pageable pages
@@ -2553,17 +2586,46 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
     CUDA_TRY(cudaEventCreate(&b.tr));
     CUDA_TRY(cudaEventCreate(&b.t1));
     CUDA_TRY(cudaEventRecord(b.t0, st));
-    if (!order.empty()) {
+    if (n_hist) {
+        ha.tasks = b.tasks.p;
+        ha.order = b.order.p;
+        ha.order_task = b.order_task.p;
+        ha.n_order = (int32_t)n_hist;
+        ha.queue = b.queue.p + 3;
+        ha.n_left = b.queue.p + 2;
+        ha.left = b.order.p + left_at;
+        ha.left_task = b.order_task.p + left_at;
+        TRY(rank_status(hist_launch(dtype, ha, S->dev.sms, hist_smem, st), "histogram kernel launch"));
+    }
+    if (n_stream) {
+        sa.tasks = b.tasks.p;
+        sa.order = b.order.p + n_hist;
+        sa.order_task = b.order_task.p + n_hist;
+        sa.n_order = (int32_t)n_stream;
+        sa.queue = b.queue.p + 1;
+        sa.n_left = b.queue.p + 2;
+        sa.left = b.order.p + left_at;
+        sa.left_task = b.order_task.p + left_at;
+        sa.dk_global = b.dk.p;
+        sa.dg_global = b.dg.p;
+        sa.slice = r.slice;
+        auto launch = dtype == HPDEX_FLOAT32 ? stream_launch_f32 : stream_launch_f64;
+        TRY(rank_status(launch(sa, std::min(S->dev.sms, (int)n_stream), stream_smem, st), "stream kernel launch"));
+    }
+    if (n_items) {
         RankArgs a{};
         a.tasks = b.tasks.p;
-        a.order = b.order.p;
-        a.order_task = b.order_task.p;
-        a.n_order = (int32_t)order.size();
+        a.order = b.order.p + left_at;
+        a.order_task = b.order_task.p + left_at;
+        a.n_order = (int32_t)n_rank;
+        a.n_order_dev = b.queue.p + 2;
         a.queue = b.queue.p;
         a.single_gene = -1;
-        bool any_int = false;  // the histogram variant when a query's matrix may hold integers
-        for (auto* q : b.q) any_int = any_int || S->mats[(size_t)q->matrix]->has_int_cols;
-        a.no_histogram = any_int ? 0 : 1;
+        // the histogram variant, which costs float genes 12%, only where integer genes are all it
+        // can get
+        bool all_int = true;
+        for (auto* q : b.q) all_int = all_int && S->mats[(size_t)q->matrix]->has_int_cols;
+        a.no_histogram = all_int ? 0 : 1;
         for (const RankTask& t : tasks) a.any_compact |= t.compact_decode;
         set_layout_args(a, r, GL, b.dk.p, b.dg.p, b.ek.p, b.eg.p, b.acc.p, b.cnt.p);
         TRY(rank_status(rank_launch(dtype, a, r.grid, r.smem, st), "rank kernel launch"));
