@@ -850,8 +850,14 @@ size_t stream_layout(const DeviceInfo& dev, int dtype, int G, const RankLayout& 
 
 // The histogram kernel's shared memory: kHistCTAs to an SM, fewer where 64 values of every group
 // need more, down to one; 0 when not even 8 values of every group fit (or the group ids are 32-bit).
-size_t hist_layout(const DeviceInfo& dev, int G, const RankLayout& r, HistArgs* a) {
-    if (!r.acc_in) return 0;
+// Its CTAs are slower with a gene than the rank kernel's (384 threads to 1,024; a gene's groups
+// take their time one after the other), so it takes launches of many genes: `genes` at least 3 to
+// an SM, and more in proportion to the groups. Rank kernel / histogram kernel time: 2,000 genes of
+// 16,000 cells 2.3 (50 groups), 1.8 (120), 1.4 (200), 1.2 (332), 0.8 (500); 500 genes 1.3, 0.8,
+// 0.6, 0.8, 0.6; 200 genes 1.0, 0.7, 0.8, 0.6, 0.5; 1,000 genes of 50,000 cells 1.3, 0.9, 0.95, 1.0,
+// 0.8.
+size_t hist_layout(const DeviceInfo& dev, int G, long long genes, const RankLayout& r, HistArgs* a) {
+    if (!r.acc_in || genes * 16 < (long long)dev.sms * std::max(48, G)) return 0;
     for (int ctas = kHistCTAs; ctas >= 1; --ctas) {
         const size_t room = std::min(dev.smem_per_sm / ctas - dev.smem_reserved, dev.smem_optin) - 2048;
         const size_t acc = hist_acc_bytes(G), values = ctas > 1 ? 64 : 8;
@@ -895,7 +901,7 @@ int configure_rank(hpdex_plan* p) {
     a.any_compact = t.compact_decode;
     set_layout_args(a, r, G, p->dk.p, p->dg.p, p->ek.p, p->eg.p, p->acc.p, p->cnt.p);
 
-    p->hist_smem = m->has_int_cols ? hist_layout(m->dev, G, r, &p->ha) : 0;
+    p->hist_smem = m->has_int_cols ? hist_layout(m->dev, G, m->n_cols, r, &p->ha) : 0;
     if (p->hist_smem) {
         TRY(p->left.alloc(std::max<long long>(m->n_cols, 1)));
         HistArgs& h = p->ha;
@@ -2526,7 +2532,10 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
     // stream kernel, the others to the rank kernel
     HistArgs ha{};
     StreamArgs sa{};
-    const size_t hist_smem = hist_layout(S->dev, GL, r, &ha);
+    long long int_genes = 0;
+    for (ServerQuery* q : b.q)
+        if (S->mats[(size_t)q->matrix]->has_int_cols) int_genes += S->mats[(size_t)q->matrix]->n_cols;
+    const size_t hist_smem = hist_layout(S->dev, GL, int_genes, r, &ha);
     const size_t stream_smem = stream_layout(S->dev, dtype, GL, r, &sa);
     std::vector<int32_t> order[3];
     std::vector<uint16_t> order_task[3];
@@ -2621,11 +2630,14 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
         a.n_order_dev = b.queue.p + 2;
         a.queue = b.queue.p;
         a.single_gene = -1;
-        // the histogram variant, which costs float genes 12%, only where integer genes are all it
-        // can get
-        bool all_int = true;
-        for (auto* q : b.q) all_int = all_int && S->mats[(size_t)q->matrix]->has_int_cols;
-        a.no_histogram = all_int ? 0 : 1;
+        // the histogram variant costs float genes 12%: only where the integer genes are this
+        // kernel's, or all that is left for it
+        bool all_int = true, any_int = false;
+        for (auto* q : b.q) {
+            all_int = all_int && S->mats[(size_t)q->matrix]->has_int_cols;
+            any_int = any_int || S->mats[(size_t)q->matrix]->has_int_cols;
+        }
+        a.no_histogram = (n_hist ? all_int : any_int) ? 0 : 1;
         for (const RankTask& t : tasks) a.any_compact |= t.compact_decode;
         set_layout_args(a, r, GL, b.dk.p, b.dg.p, b.ek.p, b.eg.p, b.acc.p, b.cnt.p);
         TRY(rank_status(rank_launch(dtype, a, r.grid, r.smem, st), "rank kernel launch"));

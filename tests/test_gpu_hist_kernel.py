@@ -8,6 +8,14 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
+def _sms():
+    import ctypes
+    from hpdex_gb300 import _lib
+    n = ctypes.c_int32()
+    _lib.check(_lib.lib().hpdex_device_sm_count(ctypes.byref(n)))
+    return n.value
+
+
 @pytest.mark.parametrize("zero", ["none", "min", "mix"])
 @pytest.mark.parametrize("dtype", [np.int8, np.uint16, np.int32, np.float32, np.float64, np.int64])
 @pytest.mark.parametrize("T", [1, 7, 49, 255, 1_000, 3_000])
@@ -33,6 +41,12 @@ def test_hist_kernel_equals_bucket_path(T, dtype, zero):
         for k in (0, 1, 2, 255, 257, 4_001):
             cols.append(rng.integers(1, 9, k).astype(dtype))
             rows.append(np.sort(rng.permutation(n_rows)[:k]))
+    # enough genes for the launch to choose the kernel (short ones, but under none)
+    filler = 3 * _sms() * max(48, T + 1) // 48 if T < 300 else 0
+    for k in range(filler):
+        n = 2 * (T + 1) if zero == "none" else int(rng.integers(0, 90))
+        cols.append(rng.integers(1, 5, n).astype(dtype))
+        rows.append(np.arange(n))
     data, indices = np.concatenate(cols), np.concatenate(rows).astype(np.int64)
     indptr = np.concatenate([[0], np.cumsum([x.size for x in cols])]).astype(np.int64)
     gid = rng.integers(-1, T + 1, n_rows).astype(np.int32)
