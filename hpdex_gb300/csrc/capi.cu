@@ -161,6 +161,7 @@ __global__ void narrow_rows_kernel(const long long* in, int32_t* out, long long 
 // kUploadCTAs CTAs of 1024 threads, four elements in flight per thread, keep the host link busy
 // from a few SMs while the persistent rank kernel of the previous chunk holds the others.
 constexpr int kUploadCTAs = 24;
+constexpr int kMatrixUploadCTAs = 76;  // of a resident matrix's upload, with the SMs to itself
 template <class V, class R>
 __global__ void __launch_bounds__(1024) upload_chunk_kernel(const V* __restrict__ hv, const R* __restrict__ hr,
                                                             V* __restrict__ dv, int32_t* __restrict__ dr,
@@ -546,7 +547,7 @@ struct KeyRangeLaunch {
 template <class V>
 struct UploadLaunch {  // one chunk, straight from the host arrays (see upload_chunk_kernel)
     static int run(const void* hv, const int64_t* hr64, const int32_t* hr32, void* dv, int32_t* dr,
-                   long long n, long long n_rows, cudaStream_t s) {
+                   long long n, long long n_rows, int ctas, cudaStream_t s) {
         if (n == 0) return HPDEX_OK;
         // quads from the first entry whose device row id is 16-byte aligned, when the other
         // three arrays are aligned to their quads there too (numpy's arrays are, at any chunk
@@ -560,16 +561,16 @@ struct UploadLaunch {  // one chunk, straight from the host arrays (see upload_c
         const bool quad = n >= lead + 4 && aligned(hv, sizeof(V), qv) && aligned(dv, sizeof(V), qv) &&
                           aligned(hr32 ? (const void*)hr32 : (const void*)hr64, hr32 ? 4 : 8, qr);
         if (quad && hr32)
-            upload_chunk_quad_kernel<V, int32_t><<<kUploadCTAs, 1024, 0, s>>>(
+            upload_chunk_quad_kernel<V, int32_t><<<ctas, 1024, 0, s>>>(
                 static_cast<const V*>(hv), hr32, static_cast<V*>(dv), dr, n, n_rows, lead);
         else if (quad)
-            upload_chunk_quad_kernel<V, int64_t><<<kUploadCTAs, 1024, 0, s>>>(
+            upload_chunk_quad_kernel<V, int64_t><<<ctas, 1024, 0, s>>>(
                 static_cast<const V*>(hv), hr64, static_cast<V*>(dv), dr, n, n_rows, lead);
         else if (hr32)
-            upload_chunk_kernel<V, int32_t><<<kUploadCTAs, 1024, 0, s>>>(
+            upload_chunk_kernel<V, int32_t><<<ctas, 1024, 0, s>>>(
                 static_cast<const V*>(hv), hr32, static_cast<V*>(dv), dr, n, n_rows);
         else
-            upload_chunk_kernel<V, int64_t><<<kUploadCTAs, 1024, 0, s>>>(
+            upload_chunk_kernel<V, int64_t><<<ctas, 1024, 0, s>>>(
                 static_cast<const V*>(hv), hr64, static_cast<V*>(dv), dr, n, n_rows);
         CUDA_TRY(cudaGetLastError());
         return HPDEX_OK;
@@ -668,13 +669,27 @@ int upload_matrix(hpdex_matrix* m, const void* data, const int64_t* indices, con
     TRY(m->data.alloc(std::max<size_t>(1, (size_t)m->nnz * vs)));
     TRY(m->rows.alloc(std::max<long long>(1, m->nnz)));
     TRY(m->indptr.alloc((size_t)m->n_cols + 1));
-    // values and int32 row ids may be host or device memory (hpdex_matrix_create_device)
-    if (m->nnz) CUDA_TRY(cudaMemcpy(m->data.p, data, (size_t)m->nnz * vs, cudaMemcpyDefault));
+    // values and int32 row ids may be host or device memory (hpdex_matrix_create_device). Where the
+    // device reaches pageable host memory, a kernel reads them there in 16-byte words and narrows
+    // the row ids on the way: group means of 3.5e7 entries (425 MB) 2.75 to 6 ms with the driver's
+    // copies of pageable memory, from process to process, 2.5 ms so (24 to 304 CTAs alike).
+    cudaPointerAttributes where{};
+    const bool on_device = m->nnz && cudaPointerGetAttributes(&where, data) == cudaSuccess &&
+                           (where.type == cudaMemoryTypeDevice || where.type == cudaMemoryTypeManaged);
+    cudaGetLastError();
+    const bool kernel_upload = m->dev.pageable_access && !on_device && m->nnz > 0;
+    if (kernel_upload)
+        TRY(dispatch_dtype<UploadLaunch>(m->dtype, data, indices, indices32, static_cast<void*>(m->data.p), m->rows.p,
+                                         m->nnz, m->n_rows, kMatrixUploadCTAs, (cudaStream_t)0));
+    else if (m->nnz)
+        CUDA_TRY(cudaMemcpy(m->data.p, data, (size_t)m->nnz * vs, cudaMemcpyDefault));
     CUDA_TRY(cudaMemcpy(m->indptr.p, indptr, sizeof(int64_t) * ((size_t)m->n_cols + 1),
                         cudaMemcpyHostToDevice));
     // row ids: int64 -> int32 through a bounded staging buffer
     const long long chunk = 1ll << 24;
-    if (m->nnz && indices32) {
+    if (kernel_upload) {
+        CUDA_TRY(cudaDeviceSynchronize());
+    } else if (m->nnz && indices32) {
         CUDA_TRY(cudaMemcpy(m->rows.p, indices32, sizeof(int32_t) * (size_t)m->nnz, cudaMemcpyDefault));
     } else if (m->nnz) {
         DevBuf<long long> stage;
@@ -2139,7 +2154,7 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
             TRY(dispatch_dtype<UploadLaunch>(dtype, static_cast<const void*>(static_cast<const unsigned char*>(data) + p0 * vs),
                                              idx32 ? nullptr : indices + p0, idx32 ? indices32 + p0 : nullptr,
                                              static_cast<void*>(m->data.p + p0 * vs), m->rows.p + p0, nk,
-                                             (long long)n_rows, sx));
+                                             (long long)n_rows, kUploadCTAs, sx));
             CUDA_TRY(cudaEventRecord(r.ev[2 * j], sx));
             return HPDEX_OK;
         }
