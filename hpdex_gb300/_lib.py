@@ -202,15 +202,15 @@ def result_array(shape):
 
 
 def fetched_array(shape):
-    """A float64 array for results copied from the device: page-locked from 1 MB on, where the
-    faults of fresh pages cost most of the call (the screen's 64 MB of results: 3.5 against 12-18
-    ms with ordinary arrays); ordinary below, where acquiring a buffer costs more than it saves
-    (0.8 MB results: 285 against 277 us)."""
+    """A float64 array for results copied from the device: page-locked from 16 MB on, where the
+    allocator maps fresh pages for every array and their faults cost most of the call (the
+    screen's 64 MB of results: 3.5 against 12-18 ms with ordinary arrays); ordinary below, where
+    acquiring a buffer costs 3 us more than it saves (two arrays of 1.3 to 13 MB)."""
     import numpy as np
     n = 1
     for d in shape:
         n *= int(d)
-    return result_array(shape) if 8 * n >= 1 << 20 else np.empty(shape, np.float64)
+    return result_array(shape) if 8 * n >= 1 << 24 else np.empty(shape, np.float64)
 
 
 def bh_fdr(p):
