@@ -1019,9 +1019,14 @@ int run_exact(hpdex_plan* p, cudaStream_t s) {
     if (dense_pairs) {
         TRY(p->pair_mark.alloc((size_t)(H * W)));
         CUDA_TRY(cudaMemsetAsync(p->pair_mark.p, 0, (size_t)(H * W), s));
-        const int g = (int)std::min<long long>((n + 255) / 256, (long long)p->m->dev.sms * 8);
-        exact_mark_pairs_kernel<<<g, 256, 0, s>>>(p->n1.p, p->n2.p, n, (int32_t)C, (int32_t)H,
-                                                  (int32_t)W, p->pair_mark.p);
+        const int gx = (int)std::min<long long>((C + 255) / 256, 1024);
+        const int gy = (int)std::max<long long>(1, std::min<long long>(T, (long long)p->m->dev.sms * 8 / gx));
+        if (H * W <= 24 * 1024)
+            exact_mark_pairs_kernel<true><<<dim3(gx, gy), 256, (size_t)(H * W), s>>>(
+                p->n1.p, p->n2.p, (int32_t)T, (int32_t)C, (int32_t)H, (int32_t)W, p->pair_mark.p);
+        else
+            exact_mark_pairs_kernel<false><<<dim3(gx, gy), 256, 0, s>>>(
+                p->n1.p, p->n2.p, (int32_t)T, (int32_t)C, (int32_t)H, (int32_t)W, p->pair_mark.p);
         CUDA_TRY(cudaGetLastError());
         std::vector<unsigned char> mark((size_t)(H * W));
         CUDA_TRY(cudaMemcpyAsync(mark.data(), p->pair_mark.p, mark.size(), cudaMemcpyDeviceToHost, s));
@@ -1057,7 +1062,7 @@ int run_exact(hpdex_plan* p, cudaStream_t s) {
     }
     const int np = (int)pairs.size();
     std::vector<long long> hn1(np), hn2(np), hoff(np), hwoff(np);
-    long long tot = 0, wtot = 0;
+    long long tot = 0, wtot = 0, largest = 0;  // largest: n1 * n2 of any pair
     for (auto& kv : pairs) {
         const int i = kv.second;
         hn1[i] = kv.first.first;
@@ -1066,6 +1071,7 @@ int run_exact(hpdex_plan* p, cudaStream_t s) {
         if (umax > (1ll << 26))
             return fail(HPDEX_ERR_UNSUPPORTED,
                         "method='exact': n1*n2 = %lld exceeds the exact-table limit 2^26", umax);
+        largest = std::max(largest, umax);
         hoff[i] = tot;
         tot += 2 * (umax + 1);
         hwoff[i] = wtot;
@@ -1108,7 +1114,11 @@ int run_exact(hpdex_plan* p, cudaStream_t s) {
     if (np > 0) {
         if (p->opt.exact_variant == HPDEX_EXACT_MWU_NULL)
             exact_null_table_kernel<256><<<np, 256, 0, s>>>(et);
-        else
+        else if (largest < kExactSmall) {
+            CUDA_TRY(cudaFuncSetAttribute(exact_reference_table_small_kernel,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExactSmallSmem));
+            exact_reference_table_small_kernel<<<np, 1024, kExactSmallSmem, s>>>(et);
+        } else
             exact_reference_table_kernel<256><<<np, 256, 0, s>>>(et);
         CUDA_TRY(cudaGetLastError());
         TRY(p->pair_recip.alloc((size_t)np));
@@ -1137,8 +1147,9 @@ int run_exact(hpdex_plan* p, cudaStream_t s) {
     a.offset = p->pair_off.p;
     a.tables = p->tables.p;
     a.recip = p->pair_recip.p;
-    const int grid = (int)std::min<long long>((n + 255) / 256, (long long)p->m->dev.sms * 8);
-    mwu_pvalue_exact_kernel<<<grid, 256, 0, s>>>(a);
+    const int gx = (int)std::min<long long>((C + 255) / 256, 1024);
+    const int gy = (int)std::max<long long>(1, std::min<long long>(T, (long long)p->m->dev.sms * 8 / gx));
+    mwu_pvalue_exact_kernel<<<dim3(gx, gy), 256, 0, s>>>(a);
     CUDA_TRY(cudaGetLastError());
     return HPDEX_OK;
 }
