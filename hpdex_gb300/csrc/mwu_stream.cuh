@@ -10,18 +10,20 @@
 //     (c0+s)^3 - (c0+s) - (c0^3 - c0) to B[g]. Every element adds the share it would have alone
 //     (s = 1), 3 c0^2 + 3 c0; pairs with s > 1 add the rest, 3 c0 (s^2 - s) + s^3 - s, once. They
 //     are found by hashing: a bitmap marks the cells that (x, g) hits and a second one those hit
-//     more than once; a second pass over the targets counts the elements of such cells (repeats,
-//     and the few pairs that share a cell) in a table, in as many hash partitions as it needs.
+//     more than once; a second pass over the targets collects the elements of such cells (repeats,
+//     and the few pairs that share a cell) and counts them in a table, in as many hash partitions
+//     as it needs.
 // The work per entry is the same for 37 groups of 400 elements and 1,500 of 20, and none of it
 // depends on a slab of the gene fitting in shared memory, which holds the sorted reference, the
 // accumulators and the table. A gene whose reference does not fit, or whose reference values
 // crowd a bucket, is listed for mwu_rank_kernel, launched behind this one.
 //
 // It gains where values seldom repeat: there mwu_rank_kernel resolves every bucket of several
-// values pairwise (continuous data at 60,000 entries a gene: 5 times its time), while here only
+// values pairwise (continuous data at 60,000 entries a gene: 5 times the time), while here only
 // the first pass over a gene is bound by memory and the rest by instruction issue. Where a few
 // values hold most elements its second pass costs more than the one-value buckets of
-// mwu_rank_kernel (a log1p-CP10k screen: 3.6 against 3.2 ms). column_ties_kernel and the plan
+// mwu_rank_kernel (1,000 genes of 10,000 entries and 20 groups, 100 steps of a normal: 0.31 against
+// 0.21 ms). column_ties_kernel and the plan
 // (stream_genes) divide the genes.
 #pragma once
 #include "mwu_rank.cuh"
@@ -213,12 +215,15 @@ __global__ void __launch_bounds__(128) column_ties_kernel(const V* data, const i
 //   reference  counted into buckets, scattered, ordered inside each bucket; equal values form runs
 //   targets    four per thread and step: two reads of the bucket table, one of the bucket's first
 //              value and run, adds to the group's sums, one bit of the bitmap
-//   repeats    only if some cell was hit twice
+//   repeats    only if some cell was hit twice: the elements of such cells are first moved together,
+//              then counted with whole warps (counted where they stood, a few lanes at a time, a
+//              screen on this kernel took 3.50 ms, now 2.90, exact mode's data 2.10, now 2.01)
 //   finalize   as in mwu_rank_kernel; p-values during the next gene's target pass
 // Bound by instruction issue (2.4 of 4 a cycle) with the shared-memory atomics next: 512 or 768
 // threads, or two CTAs' worth of registers, lose more to latency than they gain. Rank sums
 // without the p-values of exact mode 4.94 -> 2.10 ms (60,000 x 4,000 dense, 1,500 groups of 3-40:
-// 9% -> 14% of the copy bandwidth), dense doubles (20,011 x 1,501, 37 groups) 2.07 -> 0.68 ms.
+// 9% -> 14% of the copy bandwidth), dense doubles (20,011 x 1,501, 37 groups) 2.07 -> 0.68 ms; with
+// the repeats moved together 2.01 and 0.62.
 template <class V, int NT>
 __global__ void __launch_bounds__(NT, 1) mwu_stream_kernel(const StreamArgs a) {
     using K = typename Val<V>::Key;
@@ -485,24 +490,24 @@ __global__ void __launch_bounds__(NT, 1) mwu_stream_kernel(const StreamArgs a) {
             if (ties)
                 for (uint32_t i = tid; i < half / 8u; i += NT) reinterpret_cast<uint4*>(x0)[i] = make_uint4(0u, 0u, 0u, 0u);
             __syncthreads();
+            auto load = [&](uint32_t at, K* key, uint2& g) {
+                if (at < ntar) {
+                    if constexpr (sizeof(K) == 4) {
+                        const uint4 x = *reinterpret_cast<const uint4*>(dk + at);
+                        key[0] = x.x; key[1] = x.y; key[2] = x.z; key[3] = x.w;
+                    } else {
+                        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(dk + at);
+                        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(dk + at + 2);
+                        key[0] = x.x; key[1] = x.y; key[2] = y.x; key[3] = y.y;
+                    }
+                    g = *reinterpret_cast<const uint2*>(dg + at);
+                }
+            };
             // the decoded targets, four neighbours per thread (groups beyond the last: 0), the next
             // four in flight; the first `skip` warps have other work
             auto stream = [&](int skip, auto f) {
                 const uint32_t step = 4u * (uint32_t)(NT - 32 * skip);
                 uint32_t i = 4u * (uint32_t)(tid - 32 * skip);
-                auto load = [&](uint32_t at, K* key, uint2& g) {
-                    if (at < ntar) {
-                        if constexpr (sizeof(K) == 4) {
-                            const uint4 x = *reinterpret_cast<const uint4*>(dk + at);
-                            key[0] = x.x; key[1] = x.y; key[2] = x.z; key[3] = x.w;
-                        } else {
-                            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(dk + at);
-                            const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(dk + at + 2);
-                            key[0] = x.x; key[1] = x.y; key[2] = y.x; key[3] = y.y;
-                        }
-                        g = *reinterpret_cast<const uint2*>(dg + at);
-                    }
-                };
                 K ka[4], kb[4];
                 uint2 ga = make_uint2(0u, 0u), gb = make_uint2(0u, 0u);
                 auto take = [&](K* key, const uint2& gp) {
@@ -619,11 +624,48 @@ __global__ void __launch_bounds__(NT, 1) mwu_stream_kernel(const StreamArgs a) {
                 // pair sharing it, of which n^2 / 2 cells are expected
                 const float share = 0.5f * (float)ntar * (float)ntar / (float)cells;
                 const float want = 1.1f * ((float)s_cells + fminf((float)s_hits, share)) + 64.0f;
-                // the table beside the second bitmap (the first is not needed any more), at most three
-                // quarters full
-                const bool behind = xbytes - 2u * half > half;
-                PairTable table{reinterpret_cast<unsigned long long*>(x0 + (behind ? 2u * half : 0u)), 0u};
-                const uint32_t room = ((behind ? xbytes - 2u * half : half) / 16u) * 2u;
+                // The elements of cells hit more than once, each warp's to the front of its own part
+                // of the slice (never ahead of what it has read), so that the lanes that count
+                // below are all busy: one element in six of a screen's, too few in any warp.
+                constexpr uint32_t W = NT / 32;
+                const uint32_t seg = (ntar + 128u * W - 1u) / (128u * W) * 128u;
+                const uint32_t s0 = min(ntar, (uint32_t)warp * seg), s1 = min(ntar, s0 + seg);
+                uint32_t found = s0;
+                {
+                    K key[4] = {}, next[4] = {};
+                    uint2 gp = make_uint2(0u, 0u), gn = make_uint2(0u, 0u);
+                    const unsigned below = (1u << lane) - 1u;
+                    load(s0 + 4u * lane, key, gp);
+                    for (uint32_t t = s0; t < s1; t += 128u) {
+                        const uint32_t i = t + 4u * lane;
+                        if (t + 128u < s1) load(i + 128u, next, gn);
+                        const uint32_t g[4] = {gp.x & 0xffffu, gp.x >> 16, gp.y & 0xffffu, gp.y >> 16};
+                        uint32_t cell[4], w[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            cell[k] = __umulhi(pair_hash(key[k], g[k]), cells);
+                            w[k] = lds(hit_at + half + 4u * (cell[k] >> 5));
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const bool on = i + k < ntar && ((w[k] >> (cell[k] & 31u)) & 1u);
+                            const unsigned m = __ballot_sync(0xffffffffu, on);
+                            if (on) {
+                                const uint32_t o = found + __popc(m & below);
+                                dk[o] = key[k];
+                                dg[o] = (GT)g[k];
+                            }
+                            found += __popc(m);
+                        }
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) key[k] = next[k];
+                        gp = gn;
+                    }
+                }
+                // the table in the place of the bitmaps, at most three quarters full
+                PairTable table{reinterpret_cast<unsigned long long*>(x0), 0u};
+                const uint32_t room = (xbytes / 16u) * 2u;
                 uint32_t parts = 1;
                 while (want > 0.75f * (float)room * (float)parts && parts < 64u) parts *= 2u;
                 table.n = min(room, ((uint32_t)(2.0f * want) / parts + 32u) & ~1u);
@@ -631,20 +673,12 @@ __global__ void __launch_bounds__(NT, 1) mwu_stream_kernel(const StreamArgs a) {
                     __syncthreads();
                     for (uint32_t p = tid; p < table.n / 2u; p += NT) reinterpret_cast<uint4*>(table.slot)[p] = make_uint4(0u, 0u, 0u, 0u);
                     __syncthreads();
-                    stream(0, [&](const K* key, const uint32_t* g, uint32_t i) {
-                        uint32_t h[4], cell[4], w[4];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            h[k] = pair_hash(key[k], g[k]);
-                            cell[k] = __umulhi(h[k], cells);
-                            w[k] = lds(hit_at + half + 4u * (cell[k] >> 5));
-                        }
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (((w[k] >> (cell[k] & 31u)) & 1u) && g[k] && ((h[k] >> 5) & (parts - 1u)) == q &&
-                                !pair_count<K>(table, key[k], g[k], i + k, h[k] * 0x9e3779b1u, dk))
-                                s_bad = 1u;
-                    });
+                    for (uint32_t i = s0 + lane; i < found; i += 32u) {
+                        const K key = dk[i];
+                        const uint32_t g = dg[i], h = pair_hash(key, g);
+                        if (((h >> 5) & (parts - 1u)) == q && !pair_count<K>(table, key, g, i, h * 0x9e3779b1u, dk))
+                            s_bad = 1u;
+                    }
                     __syncthreads();
                     if (s_bad) return;
                     // pairs counted more than once
