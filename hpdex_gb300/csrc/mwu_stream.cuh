@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(128) column_ties_kernel(const V* data, const i
 // threads, or two CTAs' worth of registers, lose more to latency than they gain. Rank sums
 // without the p-values of exact mode 4.94 -> 2.10 ms (60,000 x 4,000 dense, 1,500 groups of 3-40:
 // 9% -> 14% of the copy bandwidth), dense doubles (20,011 x 1,501, 37 groups) 2.07 -> 0.68 ms; with
-// the repeats moved together 2.01 and 0.62.
+// the repeats moved together 2.01 and 0.62, with more buckets 1.78 (17% of the copy bandwidth) and 0.62.
 template <class V, int NT>
 __global__ void __launch_bounds__(NT, 1) mwu_stream_kernel(const StreamArgs a) {
     using K = typename Val<V>::Key;
@@ -308,9 +308,12 @@ __global__ void __launch_bounds__(NT, 1) mwu_stream_kernel(const StreamArgs a) {
             kmin = kz < kmin ? kz : kmin;
             kmax = kz > kmax ? kz : kmax;
         }
-        // about two buckets per expected reference element
-        const float expect = 2.0f * (float)nraw * (float)tk->group_rows[0] / (float)max(1u, nrows);
-        int nbl = 6;
+        // four buckets per expected reference element, at least 2,048 (two to a thread): values crowd, so
+        // that with two, and 64 at least, a target walked past the values before its own (exact
+        // mode, 40 reference cells: 2.01 ms, now 1.78; 8,192 for every gene 1.81 and the screen 1%
+        // slower for the longer clear and scan)
+        const float expect = 4.0f * (float)nraw * (float)tk->group_rows[0] / (float)max(1u, nrows);
+        int nbl = 11;
         while (nbl < a.nb_max_log2 && (float)(1u << nbl) < expect) ++nbl;
         const int NB = 1 << nbl;
         for (int g = tid; g < GL; g += NT) { A[g] = 0ull; B[g] = 0ull; nz[g] = 0u; ng[g] = 0u; b32s[g] = 0u; }
