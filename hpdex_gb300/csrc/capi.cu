@@ -409,9 +409,10 @@ struct hpdex_matrix {
     DevBuf<uint32_t> col_has_zero;
     std::vector<long long> col_nnz;  // host copy for scheduling
     long long max_col_nnz = 0;
-    // resident float matrices whose long columns seldom repeat their values: which columns take the
-    // stream kernel (else empty)
+    // resident float matrices: which columns may take the stream kernel (kStreamAny, kStreamGroups;
+    // empty: too few), and whether those of kStreamAny hold nearly all entries
     std::vector<uint8_t> col_stream;
+    bool stream_any = false;
     bool has_int_cols = true;  // some column stores only small integers (launches then use the
                                // rank kernel with the histogram path)
     DeviceInfo dev;
@@ -593,11 +594,21 @@ struct MeanLaunch {  // smem 0: accumulators in global memory
 
 // Which genes take the stream kernel: those of at least kStreamMinEntries entries whose values
 // seldom repeat (a gene of 1,024 entries: 1.13 of the rank kernel's speed there, 20 groups; of 500:
-// 0.98, 100 groups), in a matrix where they hold kStreamMinPercent of the entries: the two kernels
+// 0.98, 100 groups), where they hold kStreamMinPercent of the entries: the two kernels
 // run one after the other, each with a tail of its own (half the genes of a 100,000 x 2,000 log
-// matrix on each: 200 + 410 us, all on the rank kernel 430).
+// matrix on each: 200 + 410 us, all on the rank kernel 430). Plans of more than kStreamManyGroups
+// groups, whose (value, group) pairs repeat less than the values do, take it up to five values
+// in eight repeating, and then for short genes as well. Rank kernel / stream kernel time at
+// 500, 100, 20 and 1 targets: one value in three repeating, 10,000 entries a gene, 1.04, 1.11,
+// 0.95, 0.87, and 50,000 entries 1.21, 1.07, 0.95, 1.00; two in three, 10,000 entries, 0.95,
+// 0.90, 0.75, 0.78; the log1p-CP10k screen (500) 3.14 / 2.90 ms. The gain is small, so no gene
+// behind it may be longer than 1/kStreamRestShare of what an SM gets (a few genes of 110,000
+// entries left of 1.8e7: 0.85 / 1.39 ms).
 constexpr long long kStreamMinEntries = 1024;
 constexpr long long kStreamMinPercent = 95;
+constexpr long long kStreamManyGroups = 100;
+constexpr long long kStreamRestShare = 16;
+constexpr uint8_t kStreamAny = 1, kStreamGroups = 2;  // values of hpdex_matrix::col_stream (0: never)
 
 // Sets m->has_int_cols from the column flags of the key-range pass: some column with finite
 // nonzero values, all of them small integers (bit 1 of col_has_zero clear).
@@ -623,14 +634,17 @@ int matrix_int_hint(hpdex_matrix* m) {
         m->has_int_cols = !(f[(size_t)c] & 2u) && lo[(size_t)c] <= hi[(size_t)c];
     if (floats && !m->has_int_cols) {
         m->col_stream.resize((size_t)C);
-        long long mine = 0, all = 0;
+        long long any = 0, groups = 0, all = 0;
         for (long long c = 0; c < C; ++c) {
             const long long n = m->col_nnz[(size_t)c];
-            m->col_stream[(size_t)c] = n >= kStreamMinEntries && !(f[(size_t)c] & 4u);
+            const bool is_long = n >= kStreamMinEntries;
+            m->col_stream[(size_t)c] = (f[(size_t)c] & 8u) ? 0 : is_long && !(f[(size_t)c] & 4u) ? kStreamAny : kStreamGroups;
             all += n;
-            if (m->col_stream[(size_t)c]) mine += n;
+            if (m->col_stream[(size_t)c] == kStreamAny) any += n;
+            if (m->col_stream[(size_t)c] && is_long) groups += n;
         }
-        if (mine == 0 || mine * 100 < all * kStreamMinPercent) m->col_stream.clear();
+        m->stream_any = any > 0 && any * 100 >= all * kStreamMinPercent;
+        if (groups == 0 || groups * 100 < all * kStreamMinPercent) m->col_stream.clear();
     }
     return HPDEX_OK;
 }
@@ -863,6 +877,19 @@ size_t stream_layout(const DeviceInfo& dev, int dtype, int G, const RankLayout& 
     return fixed + (size_t)a->region;
 }
 
+// The longest column whose reference the stream kernel is expected to hold: a longer one would be
+// read there only to be left to the rank kernel (200,000 x 1,000 log matrix, 33,000 reference
+// cells: 0.85 ms on the rank kernel, 1.4 with the genes that were left). No margin: a gene that fits
+// gains more than one that was left loses (300 dense doubles, 10,000 reference cells: 2.05 / 0.39
+// ms; 1.97 / 2.05 where all were left).
+long long stream_longest(const DeviceInfo& dev, int dtype, int G, long long ref_rows, long long n_rows) {
+    const size_t budget = std::min(dev.smem_per_sm - dev.smem_reserved, dev.smem_optin) - 2048;
+    const size_t fixed = stream_acc_bytes(G) + stream_bucket_bytes(13) + kStreamMinTable;
+    if (fixed > budget) return -1;
+    const double cap = (double)((budget - fixed) / (2 * dtype_size(dtype) + 2));
+    return (long long)(cap * (double)n_rows / (double)std::max<long long>(ref_rows, 1));
+}
+
 // The histogram kernel's shared memory: kHistCTAs to an SM, fewer where 64 values of every group
 // need more, down to one; 0 when not even 8 values of every group fit (or the group ids are 32-bit).
 // Its CTAs are slower with a gene than the rank kernel's (384 threads to 1,024; a gene's groups
@@ -956,9 +983,25 @@ int stream_genes(hpdex_plan* p, const std::vector<int32_t>& order) {
     const hpdex_matrix* m = p->m;
     p->n_stream = 0;
     if (p->stream_mode == 0 || (p->stream_mode < 0 && m->col_stream.empty())) return HPDEX_OK;
+    const long long longest = stream_longest(m->dev, m->dtype, (int)p->G, p->group_rows[0], m->n_rows);
     std::vector<int32_t> mine, rest;
-    for (const int32_t c : order)
-        (p->stream_mode == 1 || m->col_stream[(size_t)c] ? mine : rest).push_back(c);
+    auto divide = [&](uint8_t level) {  // whether it pays
+        mine.clear();
+        rest.clear();
+        long long all = 0, held = 0, rest_longest = 0;  // (held: entries of the stream kernel's long genes)
+        for (const int32_t c : order) {
+            const long long n = m->col_nnz[(size_t)c];
+            const bool fits = m->col_stream[(size_t)c] && m->col_stream[(size_t)c] <= level && n <= longest;
+            (fits ? mine : rest).push_back(c);
+            all += n;
+            if (!fits) rest_longest = std::max(rest_longest, n);
+            else if (n >= kStreamMinEntries) held += n;
+        }
+        return held > 0 && held * 100 >= all * kStreamMinPercent &&
+               (level == kStreamAny || rest_longest * kStreamRestShare * m->dev.sms <= all);
+    };
+    if (p->stream_mode == 1) mine = order;
+    else if (!(p->G > kStreamManyGroups && divide(kStreamGroups)) && !divide(kStreamAny)) return HPDEX_OK;
     if (mine.empty()) return HPDEX_OK;
     const int32_t init[4] = {0, 0, (int32_t)rest.size(), 0};
     TRY(p->left.alloc(order.size()));
@@ -2576,9 +2619,11 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
             const auto& seg = S->mat_class_start[(size_t)b.q[i]->matrix];
             const int64_t lo = seg[(size_t)(2 * k)], hi = seg[(size_t)(2 * k + 1)];
             const bool hist = hist_smem && m->has_int_cols;
+            const long long longest = stream_smem && m->stream_any
+                ? stream_longest(S->dev, dtype, GL, b.q[i]->group_rows[0], m->n_rows) : -1;
             for (int64_t j = lo; j < hi; ++j) {
                 const int32_t c = ord[(size_t)j];
-                put(hist ? 0 : stream_smem && !m->col_stream.empty() && m->col_stream[(size_t)c] ? 1 : 2, c, i);
+                put(hist ? 0 : m->col_nnz[(size_t)c] <= longest && m->col_stream[(size_t)c] == kStreamAny ? 1 : 2, c, i);
             }
         }
     const size_t n_hist = order[0].size(), n_stream = order[1].size(), n_rank = order[2].size();

@@ -178,7 +178,8 @@ __device__ __forceinline__ bool pair_count(const PairTable& t, K key, uint32_t g
 // Whether a column's values repeat: of kTieSample entries, evenly spaced over it, more than one in
 // eight equal an earlier one (a screen's columns: one in three and more; values drawn from 3,000
 // normal steps: one in nine, where the two kernels take the same time). Sets bit 2 of flags[c] for
-// the columns of at least 2 * kTieSample entries, one block each.
+// the columns of at least 2 * kTieSample entries, one block each, and bit 3 where more than five
+// in eight do (plans of many groups take columns below that).
 constexpr int kTieSample = 512;
 template <class V>
 __global__ void __launch_bounds__(128) column_ties_kernel(const V* data, const int64_t* indptr, uint32_t* flags) {
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(128) column_ties_kernel(const V* data, const i
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0 && equal > kTieSample / 8) flags[blockIdx.x] |= 4u;
+    if (threadIdx.x == 0 && equal > kTieSample / 8) flags[blockIdx.x] |= equal > 5 * kTieSample / 8 ? 12u : 4u;
 }
 
 // One 1,024-thread CTA per SM takes genes from the work queue. Per gene:
