@@ -884,9 +884,9 @@ size_t stream_layout(const DeviceInfo& dev, int dtype, int G, const RankLayout& 
 // ms; 1.97 / 2.05 where all were left).
 long long stream_longest(const DeviceInfo& dev, int dtype, int G, long long ref_rows, long long n_rows) {
     const size_t budget = std::min(dev.smem_per_sm - dev.smem_reserved, dev.smem_optin) - 2048;
-    const size_t fixed = stream_acc_bytes(G) + stream_bucket_bytes(13) + kStreamMinTable;
-    if (fixed > budget) return -1;
-    const double cap = (double)((budget - fixed) / (2 * dtype_size(dtype) + 2));
+    const size_t fixed = stream_acc_bytes(G) + stream_bucket_bytes(13);
+    if (fixed + 4 * kStreamMinTable > budget) return -1;
+    const double cap = (double)stream_ref_cap((budget - fixed) & ~(size_t)15, dtype_size(dtype));
     return (long long)(cap * (double)n_rows / (double)std::max<long long>(ref_rows, 1));
 }
 

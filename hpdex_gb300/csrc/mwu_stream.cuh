@@ -50,7 +50,14 @@ struct StreamArgs {
 };
 
 constexpr int kStreamMaxBucket = 512;    // reference elements of a bucket of several values
-constexpr uint32_t kStreamMinTable = 16u << 10;  // bytes of table a gene must have left
+constexpr uint32_t kStreamMinTable = 16u << 10;  // (a region is at least four of these)
+
+// Reference elements that a region holds: their keys twice (as read, as scattered) and the ends of
+// their runs, two paddings of 16 bytes. The bitmaps and the table come where the scattered keys
+// were: at least 2/5 of a region of 4 * kStreamMinTable bytes, the smallest a launch has.
+__host__ __device__ inline uint32_t stream_ref_cap(size_t region, size_t key_bytes) {
+    return (uint32_t)((region - 64) / (2 * key_bytes + 2));
+}
 
 // Shared memory: accumulators (28 bytes per group: A and B as in mwu_rank_kernel, the stored and
 // negative counts, and the targets' own shares of B in one word), bucket table, then the region.
@@ -338,7 +345,7 @@ __global__ void __launch_bounds__(NT, 1) mwu_stream_kernel(const StreamArgs a) {
             // ---- the entries once: reference keys to the start of the region, the stored
             // targets' (key, group) to the CTA's slice ----
             K* stage = reinterpret_cast<K*>(region);
-            const uint32_t cap = ((uint32_t)a.region - kStreamMinTable) / (2u * (uint32_t)sizeof(K) + 2u);
+            const uint32_t cap = stream_ref_cap((size_t)a.region, sizeof(K));
             {
                 // a warp's tile of 128: 4 entries per lane, neighbouring lanes on neighbouring
                 // entries (a whole tile: no bounds to test)

@@ -36,3 +36,27 @@ def test_choice_changes_nothing(steps, ref, long_rest, dtype, T):
     for other in got[1:]:
         for a, b in zip(got[0], other):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,held", [(np.float32, 19_744), (np.float64, 10_968)])
+def test_references_at_the_capacity(dtype, held):
+    """Dense genes whose references fill the stream kernel's shared memory to the last entries, and
+    exceed it (held: (230,400 - 96 - 32,800, in whole 16 bytes, - 64) / (2 * key bytes + 2))."""
+    from hpdex_gb300.resident import ResidentMatrix
+    rng = np.random.default_rng(3)
+    for ref in (held - 9, held - 1, held, held + 1, held + 9):
+        n_rows = ref + 700
+        data = (np.round(rng.standard_normal(3 * n_rows) * 3000) + 0.25) / 3000
+        indptr = np.arange(4, dtype=np.int64) * n_rows
+        gid = np.zeros(n_rows, np.int32)
+        gid[rng.permutation(n_rows)[:700]] = np.repeat([1, 2], 350)
+        m = ResidentMatrix(data.astype(dtype), np.tile(np.arange(n_rows, dtype=np.int64), 3), indptr, n_rows)
+        plan = m.plan(gid, 2, zero_handling="min")
+        got = []
+        for mode in (-1, 1, 0):
+            plan.set_stream(mode)
+            plan.run()
+            got.append([x.copy() for x in plan.download()])
+        for other in got[1:]:
+            for a, b in zip(got[0], other):
+                np.testing.assert_array_equal(a, b)
