@@ -7,7 +7,7 @@ tie and continuity corrections, two-sided asymptotic p-values. Synthetic, seeded
 One step = one DE call: per-(gene, target) U1 and P for all 500 x 8,000 tests.
   value : tests/s with the matrix resident in HBM (library layout: float32 values, int32 row
           ids, int64 column pointers, per-column key ranges), batched form (group-id
-          preparation + persistent work-queue rank kernel that also computes the p-values,
+          preparation + persistent work-queue kernel that also computes the p-values,
           replayed as one CUDA graph), device time from CUDA events recorded inside the graph
           on the launching stream. kernels_ms also times the same plan with the p-values in a
           separate kernel.
@@ -84,8 +84,8 @@ def peaks():
 
 
 def profile_figure(key):
-    """A per-launch figure of the rank kernel from the committed ncu summary, if present."""
-    path = os.path.join(ROOT, "profiles", "mwu_rank_kernel_perturb_screen.txt")
+    """A per-launch figure of the screen's kernel from the committed ncu summary, if present."""
+    path = os.path.join(ROOT, "profiles", "mwu_stream_kernel_perturb_screen.txt")
     if not os.path.exists(path):
         return None
     for line in open(path):
@@ -98,7 +98,7 @@ def profile_figure(key):
 
 
 def traffic_from_profile():
-    """DRAM bytes per rank-kernel launch (dram__bytes_read.sum + dram__bytes_write.sum)."""
+    """DRAM bytes per launch of the screen's kernel (dram__bytes_read.sum + dram__bytes_write.sum)."""
     return profile_figure("traffic_bytes_per_launch_full_workload")
 
 
@@ -472,7 +472,7 @@ def umi_leg(hbm, steps=20):
 def exact_leg(steps=3):
     """Exact-mode workload (60,000 cells x 4,000 genes dense float32 N(0,1) with per-target
     shifts, 40 reference cells, 1,500 targets of 3-40 cells, zero_handling=none): device tests/s
-    for the reference-compatible DP variant and the true-null variant (rank kernel, then the
+    for the reference-compatible DP variant and the true-null variant (stream kernel, then the
     table build and lookup), and the oracle port on a gene sample on the host."""
     from hpdex_gb300 import synthetic
     from hpdex_gb300.resident import ResidentMatrix
@@ -590,7 +590,7 @@ def run_ours(args, rank, world):
             dist.destroy_process_group()
         return 0
 
-    # the same plan with the p-values in a separate kernel after the rank kernel (context for
+    # the same plan with the p-values in a separate kernel after it (context for
     # the fused stage's gain; not timed as the metric)
     plan.set_fused_pvalues(False)
     sep = []
@@ -709,7 +709,7 @@ def run_ours(args, rank, world):
         "exact": exact,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                      "frac": achieved / hbm, "traffic": traffic,
-                     "kernel": "mwu_rank_kernel", "algorithmic_bytes": B,
+                     "kernel": "mwu_stream_kernel", "algorithmic_bytes": B,
                      "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)",
                      "issue": issue},
         "clocks": clocks,
