@@ -584,7 +584,7 @@ struct MeanLaunch {  // smem 0: accumulators in global memory
             group_mean_kernel<V, kMeanThreads><<<grid, kMeanThreads, 0, s>>>(*a);
         } else {
             auto k = group_mean_fixed_kernel<V, kMeanFixedThreads>;
-            CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CUDA_TRY(allow_max_smem(k));
             k<<<grid, kMeanFixedThreads, smem, s>>>(*a);
         }
         CUDA_TRY(cudaGetLastError());
@@ -1158,8 +1158,7 @@ int run_exact(hpdex_plan* p, cudaStream_t s) {
         if (p->opt.exact_variant == HPDEX_EXACT_MWU_NULL)
             exact_null_table_kernel<256><<<np, 256, 0, s>>>(et);
         else if (largest < kExactSmall) {
-            CUDA_TRY(cudaFuncSetAttribute(exact_reference_table_small_kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExactSmallSmem));
+            CUDA_TRY(allow_max_smem(exact_reference_table_small_kernel));
             exact_reference_table_small_kernel<<<np, 1024, kExactSmallSmem, s>>>(et);
         } else
             exact_reference_table_kernel<256><<<np, 256, 0, s>>>(et);
@@ -1328,8 +1327,8 @@ struct TransposeLaunch {
         const size_t smem = sizeof(uint32_t) * (size_t)C;
         const bool in_smem = smem <= 160 * 1024;
         if (in_smem) {
-            CUDA_TRY(cudaFuncSetAttribute(csr_block_count_kernel<true, GI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            CUDA_TRY(cudaFuncSetAttribute(csr_scatter_kernel<V, true, GI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CUDA_TRY(allow_max_smem(csr_block_count_kernel<true, GI>));
+            CUDA_TRY((allow_max_smem(csr_scatter_kernel<V, true, GI>)));
             csr_block_count_kernel<true, GI><<<nb, kTransposeThreads, smem>>>(dptr.p, dgen.p, R, rpb, (int)C, cnt.p);
         } else {
             CUDA_TRY(cudaMemset(cnt.p, 0, sizeof(uint32_t) * (size_t)nb * C));
@@ -1478,7 +1477,7 @@ int hpdex_bh_fdr(const double* p, int64_t n, double* fdr) {
     cudaStream_t s = 0;
     CUDA_TRY(cudaMemcpyAsync(k0.p, p, sizeof(double) * n, cudaMemcpyHostToDevice, s));
     CUDA_TRY(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), s));
-    CUDA_TRY(cudaFuncSetAttribute(radix_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortScatterSmem));
+    CUDA_TRY(allow_max_smem(radix_scatter_kernel));
     unsigned long long* kin = k0.p;
     unsigned long long* kout = k1.p;
     uint32_t* vin = nullptr;

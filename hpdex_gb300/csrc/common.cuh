@@ -6,6 +6,21 @@
 
 namespace hpdex {
 
+// Opts a kernel into all the dynamic shared memory that a block may have on the current device. The
+// attribute belongs to the process: set to one launch's own bytes, another thread's smaller launch
+// may lower it before the first is issued, which then fails ("too many resources requested").
+template <class F>
+inline cudaError_t allow_max_smem(F* kernel) {
+    cudaFuncAttributes fa;
+    int dev = 0, optin = 0;
+    cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
+    return e;
+}
+
 // Reference enum values (AI4Cell/hpdex src/cpp/include/mannwhitneyu.hpp:24-31).
 enum ZeroHandling : int { ZH_NONE = 0, ZH_MIN = 1, ZH_MAX = 2, ZH_MIX = 3 };
 enum Alternative : int { ALT_LESS = 0, ALT_GREATER = 1, ALT_TWO_SIDED = 2 };

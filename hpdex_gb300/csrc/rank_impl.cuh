@@ -23,7 +23,7 @@ cudaError_t HPDEX_CAT(rank_launch_, HPDEX_RANK_T)(const RankArgs& a, int grid, s
 cudaError_t HPDEX_CAT(hist_launch_, HPDEX_RANK_T)(const HistArgs& a, int sms, size_t smem,
                                                   cudaStream_t s) {
     auto k = mwu_hist_kernel<HPDEX_RANK_V, kHistThreads, kHistCTAs>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_max_smem(k);
     if (e != cudaSuccess) return e;
     int blocks = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, kHistThreads, smem);

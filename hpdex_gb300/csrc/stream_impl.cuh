@@ -11,7 +11,7 @@ namespace hpdex {
 cudaError_t HPDEX_CAT(stream_launch_, HPDEX_STREAM_T)(const StreamArgs& a, int grid, size_t smem,
                                                       cudaStream_t s) {
     auto k = mwu_stream_kernel<HPDEX_STREAM_V, kStreamThreads>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_max_smem(k);
     if (e != cudaSuccess) return e;
     k<<<grid, kStreamThreads, smem, s>>>(a);
     return cudaGetLastError();
