@@ -545,6 +545,15 @@ struct KeyRangeLaunch {
     }
 };
 
+// Whether the upload kernel may read the caller's arrays where they are: the device reaches them, and
+// they hold their elements at natural alignment. numpy has arrays that do not (views into byte
+// buffers); a misaligned load faults the GPU, the driver's copies take them.
+bool kernel_reads(const DeviceInfo& dev, int dtype, const void* data, const int64_t* indices,
+                  const int32_t* indices32) {
+    auto aligned = [](const void* p, size_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
+    return dev.pageable_access && aligned(data, dtype_size(dtype)) &&
+           (indices32 ? aligned(indices32, sizeof(int32_t)) : aligned(indices, sizeof(int64_t)));
+}
 template <class V>
 struct UploadLaunch {  // one chunk, straight from the host arrays (see upload_chunk_kernel)
     static int run(const void* hv, const int64_t* hr64, const int32_t* hr32, void* dv, int32_t* dr,
@@ -684,14 +693,14 @@ int upload_matrix(hpdex_matrix* m, const void* data, const int64_t* indices, con
     TRY(m->rows.alloc(std::max<long long>(1, m->nnz)));
     TRY(m->indptr.alloc((size_t)m->n_cols + 1));
     // values and int32 row ids may be host or device memory (hpdex_matrix_create_device). Where the
-    // device reaches pageable host memory, a kernel reads them there in 16-byte words and narrows
+    // device reaches pageable host memory (kernel_reads), a kernel reads them there in 16-byte words and narrows
     // the row ids on the way: group means of 3.5e7 entries (425 MB) 2.75 to 6 ms with the driver's
     // copies of pageable memory, from process to process, 2.5 ms so (24 to 304 CTAs alike).
     cudaPointerAttributes where{};
     const bool on_device = m->nnz && cudaPointerGetAttributes(&where, data) == cudaSuccess &&
                            (where.type == cudaMemoryTypeDevice || where.type == cudaMemoryTypeManaged);
     cudaGetLastError();
-    const bool kernel_upload = m->dev.pageable_access && !on_device && m->nnz > 0;
+    const bool kernel_upload = !on_device && m->nnz > 0 && kernel_reads(m->dev, m->dtype, data, indices, indices32);
     if (kernel_upload)
         TRY(dispatch_dtype<UploadLaunch>(m->dtype, data, indices, indices32, static_cast<void*>(m->data.p), m->rows.p,
                                          m->nnz, m->n_rows, kMatrixUploadCTAs, (cudaStream_t)0));
@@ -2175,7 +2184,7 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
     // where the device reaches pageable host memory, a few CTAs read each chunk straight from the
     // caller's arrays (no staging, no driver copies); else cudaMemcpyAsync (int64 row ids through
     // staging buffers, narrowed on the device)
-    const bool kernel_upload = m->dev.pageable_access;
+    const bool kernel_upload = kernel_reads(m->dev, dtype, data, indices, indices32);
     if (!idx32 && !kernel_upload)
         for (auto& b : stage) TRY(b.alloc((size_t)std::max<long long>(max_chunk, 1)));
 
