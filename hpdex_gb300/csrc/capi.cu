@@ -71,6 +71,20 @@ constexpr int kPlainStreams = 128;  // concurrent streams of the plain form (the
 constexpr int kMeanThreads = 256;
 constexpr int kMeanFixedThreads = 512;
 
+// Whether a kernel may write the caller's doubles (`bytes` > 0) at `p` because they are page-locked: the first
+// and the last byte, so that an array registered in part is not written past its registration.
+bool page_locked(const void* p, size_t bytes) {
+    const unsigned char* ends[2] = {static_cast<const unsigned char*>(p), static_cast<const unsigned char*>(p) + bytes - 1};
+    bool ok = p != nullptr && bytes > 0 && reinterpret_cast<uintptr_t>(p) % sizeof(double) == 0;
+    for (int k = 0; k < 2 && ok; ++k) {
+        cudaPointerAttributes at{};
+        ok = cudaPointerGetAttributes(&at, ends[k]) == cudaSuccess && at.type == cudaMemoryTypeHost &&
+             at.devicePointer == ends[k];
+    }
+    cudaGetLastError();
+    return ok;
+}
+
 struct DeviceInfo {
     int device = -1;
     int sms = 0;
@@ -2053,9 +2067,7 @@ int matrix_group_mean(const hpdex_matrix* m, const int32_t* group_id, int64_t n_
     TRY(grows.alloc(G));
     if (fixed) TRY(gid16.alloc(std::max<long long>(n_rows, 1)));
     // a page-locked result buffer is written by the kernel itself
-    cudaPointerAttributes at{};
-    const bool direct = cudaPointerGetAttributes(&at, out) == cudaSuccess && at.type == cudaMemoryTypeHost;
-    cudaGetLastError();
+    const bool direct = page_locked(out, sizeof(double) * (size_t)n_cols * G);
     if (!direct) TRY(dout.alloc((size_t)n_cols * G));
     if (n_rows) CUDA_TRY(cudaMemcpyAsync(gid.p, group_id, sizeof(int32_t) * n_rows, cudaMemcpyHostToDevice, 0));
     CUDA_TRY(cudaMemsetAsync(grows.p, 0, sizeof(unsigned int) * G, 0));
@@ -2300,14 +2312,8 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
     // the compute stream waits for it before the first p-value kernel.
     // Page-locked outputs (hpdex_host_buffer_acquire) are written directly on any system and
     // need no touching; pageable ones directly where the device can reach pageable memory.
-    bool pinned_out = false;
-    if (U1_out && P_out) {
-        cudaPointerAttributes a1{}, a2{};
-        if (cudaPointerGetAttributes(&a1, U1_out) == cudaSuccess &&
-            cudaPointerGetAttributes(&a2, P_out) == cudaSuccess)
-            pinned_out = a1.type == cudaMemoryTypeHost && a2.type == cudaMemoryTypeHost;
-        cudaGetLastError();
-    }
+    const size_t out_bytes = sizeof(double) * (size_t)(p->T * C);
+    const bool pinned_out = page_locked(U1_out, out_bytes) && page_locked(P_out, out_bytes);
     const bool direct = (m->dev.pageable_access || pinned_out) && U1_out && P_out;
     std::atomic<int> touched{pinned_out ? 1 : 0};
     struct Toucher {
@@ -2315,9 +2321,8 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
         ~Toucher() { if (t.joinable()) t.join(); }
     } toucher;
     if (direct && !pinned_out) {
-        const size_t bytes = sizeof(double) * (size_t)(T * C);
-        toucher.t = std::thread([U1_out, P_out, bytes, &touched] {
-            for (size_t o = 0; o < bytes; o += 4096) {
+        toucher.t = std::thread([U1_out, P_out, out_bytes, &touched] {
+            for (size_t o = 0; o < out_bytes; o += 4096) {
                 reinterpret_cast<volatile unsigned char*>(U1_out)[o] = 0;
                 reinterpret_cast<volatile unsigned char*>(P_out)[o] = 0;
             }
@@ -2655,15 +2660,10 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
     // of hpdex_host_buffer_acquire) or when the device reaches pageable memory; pageable pages
     // that were never written would fault one by one when the device writes them: touch them
     for (ServerQuery* q : b.q) {
-        bool pinned = false;
-        cudaPointerAttributes a1{}, a2{};
-        if (cudaPointerGetAttributes(&a1, q->U1_out) == cudaSuccess &&
-            cudaPointerGetAttributes(&a2, q->P_out) == cudaSuccess)
-            pinned = a1.type == cudaMemoryTypeHost && a2.type == cudaMemoryTypeHost;
-        cudaGetLastError();
+        const size_t bytes = sizeof(double) * (size_t)(q->T * S->mats[(size_t)q->matrix]->n_cols);
+        const bool pinned = page_locked(q->U1_out, bytes) && page_locked(q->P_out, bytes);
         q->direct = pinned || S->dev.pageable_access;
         if (!q->direct || pinned) continue;
-        const size_t bytes = sizeof(double) * (size_t)(q->T * S->mats[(size_t)q->matrix]->n_cols);
         for (size_t o = 0; o < bytes; o += 4096) {
             reinterpret_cast<volatile unsigned char*>(q->U1_out)[o] = 0;
             reinterpret_cast<volatile unsigned char*>(q->P_out)[o] = 0;
