@@ -2069,6 +2069,9 @@ int matrix_group_mean(const hpdex_matrix* m, const int32_t* group_id, int64_t n_
     // a page-locked result buffer is written by the kernel itself
     const bool direct = page_locked(out, sizeof(double) * (size_t)n_cols * G);
     if (!direct) TRY(dout.alloc((size_t)n_cols * G));
+    const int grid = fixed ? (int)n_cols : (int)std::min<long long>(n_cols, (long long)m->dev.sms * 4);
+    if (!fixed) TRY(acc.alloc((size_t)grid * 16 * G));
+    // (nothing is allocated behind the first launch: a failure would hand buffers in use back)
     if (n_rows) CUDA_TRY(cudaMemcpyAsync(gid.p, group_id, sizeof(int32_t) * n_rows, cudaMemcpyHostToDevice, 0));
     CUDA_TRY(cudaMemsetAsync(grows.p, 0, sizeof(unsigned int) * G, 0));
     if (n_rows) {
@@ -2094,12 +2097,7 @@ int matrix_group_mean(const hpdex_matrix* m, const int32_t* group_id, int64_t n_
     a.group_rows = grows.p;
     a.include_zeros = include_zeros;
     a.out = direct ? out : dout.p;
-    int grid = (int)n_cols;
-    if (!fixed) {
-        grid = (int)std::min<long long>(n_cols, (long long)m->dev.sms * 4);
-        TRY(acc.alloc((size_t)grid * 16 * G));
-        a.acc_global = acc.p;
-    }
+    a.acc_global = acc.p;
     TRY(dispatch_dtype<MeanLaunch>(m->dtype, &a, grid, fixed ? need : (size_t)0, (cudaStream_t)0));
     CUDA_TRY(cudaStreamSynchronize(0));
     if (!direct) CUDA_TRY(cudaMemcpy(out, dout.p, sizeof(double) * (size_t)n_cols * G, cudaMemcpyDeviceToHost));
