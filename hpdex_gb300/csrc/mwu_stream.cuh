@@ -157,10 +157,12 @@ __device__ __forceinline__ K slot_key(unsigned long long s, const K* dk) {
     if constexpr (sizeof(K) == 4) return (uint32_t)(s >> 32);
     else return dk[(uint32_t)(s >> 32)];
 }
-// Counts one element; false when the table has no room within the probe limit.
+// Counts one element; false when the table has no room within the probe limit, or (`wide`: more elements
+// are counted than a slot can hold) the pair's count leaves its 16 bits. (That count may have carried into the
+// group; every other lookup still ends, and the caller drops the table.)
 template <class K>
 __device__ __forceinline__ bool pair_count(const PairTable& t, K key, uint32_t g, uint32_t entry,
-                                           uint32_t h, const K* dk) {
+                                           uint32_t h, const K* dk, bool wide) {
     const uint32_t id = sizeof(key) == 4 ? (uint32_t)key : entry;
     const unsigned long long mine = ((unsigned long long)id << 32) | (g << 16) | 1u;
     uint32_t p = __umulhi(h, t.n);
@@ -174,7 +176,9 @@ __device__ __forceinline__ bool pair_count(const PairTable& t, K key, uint32_t g
         if constexpr (sizeof(key) == 4) same = (cur >> 16) == (mine >> 16);
         else same = (((uint32_t)cur >> 16) == g) && slot_key(cur, dk) == key;
         if (same) {
-            red_add<true>(reinterpret_cast<uint32_t*>(t.slot + p), 1u);
+            uint32_t* count = reinterpret_cast<uint32_t*>(t.slot + p);
+            if (wide) return (atomicAdd(count, 1u) & 0xffffu) != 0xffffu;
+            red_add<true>(count, 1u);
             return true;
         }
         p = p + 1u == t.n ? 0u : p + 1u;
@@ -624,17 +628,14 @@ __global__ void __launch_bounds__(NT, 1) mwu_stream_kernel(const StreamArgs a) {
             more = __reduce_add_sync(0xffffffffu, more);
             if (lane == 0 && hits) { atomicAdd(&s_hits, hits); atomicAdd(&s_cells, more); }
             __syncthreads();
-            if (ties && ntar > 0xffffu) {  // a slot counts to 65,535
-                for (int g = 1 + tid; g < G; g += NT)
-                    if (nz[g] > 0xffffu) s_bad = 1u;
-                __syncthreads();
-            }
-            if (s_bad || !ties) return;
+            if (!ties) return;
             if (s_hits) {
                 // distinct pairs to count: one per cell hit more than once and one per further
                 // pair sharing it, of which n^2 / 2 cells are expected
                 const float share = 0.5f * (float)ntar * (float)ntar / (float)cells;
                 const float want = 1.1f * ((float)s_cells + fminf((float)s_hits, share)) + 64.0f;
+                // a slot counts to 65,535; the elements counted are those of cells hit more than once
+                const bool wide = s_hits + s_cells > 0xffffu;
                 // The elements of cells hit more than once, each warp's to the front of its own part
                 // of the slice (never ahead of what it has read), so that the lanes that count
                 // below are all busy: one element in six of a screen's, too few in any warp.
@@ -687,7 +688,7 @@ __global__ void __launch_bounds__(NT, 1) mwu_stream_kernel(const StreamArgs a) {
                     for (uint32_t i = s0 + lane; i < found; i += 32u) {
                         const K key = dk[i];
                         const uint32_t g = dg[i], h = pair_hash(key, g);
-                        if (((h >> 5) & (parts - 1u)) == q && !pair_count<K>(table, key, g, i, h * 0x9e3779b1u, dk))
+                        if (((h >> 5) & (parts - 1u)) == q && !pair_count<K>(table, key, g, i, h * 0x9e3779b1u, dk, wide))
                             s_bad = 1u;
                     }
                     __syncthreads();
