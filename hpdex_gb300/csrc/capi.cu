@@ -426,6 +426,8 @@ struct hpdex_matrix {
     // resident float matrices: which columns may take the stream kernel (kStreamAny, kStreamGroups;
     // empty: too few), and whether those of kStreamAny hold nearly all entries
     std::vector<uint8_t> col_stream;
+    std::vector<float> col_repeat;   // with col_stream: how far each column repeats its values
+                                     // (column_ties_kernel)
     bool stream_any = false;
     bool has_int_cols = true;  // some column stores only small integers (launches then use the
                                // rank kernel with the histogram path)
@@ -615,17 +617,14 @@ struct MeanLaunch {  // smem 0: accumulators in global memory
     }
 };
 
-// Which genes take the stream kernel: those of at least kStreamMinEntries entries whose values
-// seldom repeat (a gene of 1,024 entries: 1.13 of the rank kernel's speed there, 20 groups; of 500:
-// 0.98, 100 groups), where they hold kStreamMinPercent of the entries: the two kernels
+// Which genes may take the stream kernel, by their values alone (hpdex_matrix::col_stream; StreamRule
+// decides for a grouping): those of at least kStreamMinEntries entries whose values seldom repeat
+// (kStreamAny), where they hold kStreamMinPercent of the entries: the two kernels
 // run one after the other, each with a tail of its own (half the genes of a 100,000 x 2,000 log
 // matrix on each: 200 + 410 us, all on the rank kernel 430). Plans of more than kStreamManyGroups
 // groups, whose (value, group) pairs repeat less than the values do, take it up to five values
-// in eight repeating, and then for short genes as well. Rank kernel / stream kernel time at
-// 500, 100, 20 and 1 targets: one value in three repeating, 10,000 entries a gene, 1.04, 1.11,
-// 0.95, 0.87, and 50,000 entries 1.21, 1.07, 0.95, 1.00; two in three, 10,000 entries, 0.95,
-// 0.90, 0.75, 0.78; the log1p-CP10k screen (500) 3.14 / 2.90 ms. The gain is small, so no gene
-// behind it may be longer than 1/kStreamRestShare of what an SM gets (a few genes of 110,000
+// in eight repeating (kStreamGroups), and then for short genes as well. The gain is small there (the
+// log1p-CP10k screen of 500 targets 3.14 / 2.90 ms), so no gene behind it may be longer than 1/kStreamRestShare of what an SM gets (a few genes of 110,000
 // entries left of 1.8e7: 0.85 / 1.39 ms).
 constexpr long long kStreamMinEntries = 1024;
 constexpr long long kStreamMinPercent = 95;
@@ -641,11 +640,13 @@ int matrix_int_hint(hpdex_matrix* m) {
     m->has_int_cols = false;
     if (C == 0) return HPDEX_OK;
     const bool floats = m->dtype == HPDEX_FLOAT32 || m->dtype == HPDEX_FLOAT64;
+    DevBuf<float> repeat;
     if (floats) {
+        TRY(repeat.alloc((size_t)C));
         if (m->dtype == HPDEX_FLOAT32)
-            column_ties_kernel<float><<<(int)C, 128>>>(reinterpret_cast<const float*>(m->data.p), m->indptr.p, m->col_has_zero.p);
+            column_ties_kernel<float><<<(int)C, 128>>>(reinterpret_cast<const float*>(m->data.p), m->indptr.p, m->col_has_zero.p, repeat.p);
         else
-            column_ties_kernel<double><<<(int)C, 128>>>(reinterpret_cast<const double*>(m->data.p), m->indptr.p, m->col_has_zero.p);
+            column_ties_kernel<double><<<(int)C, 128>>>(reinterpret_cast<const double*>(m->data.p), m->indptr.p, m->col_has_zero.p, repeat.p);
         CUDA_TRY(cudaGetLastError());
     }
     std::vector<uint32_t> f((size_t)C);
@@ -656,6 +657,8 @@ int matrix_int_hint(hpdex_matrix* m) {
     for (long long c = 0; c < C && !m->has_int_cols; ++c)
         m->has_int_cols = !(f[(size_t)c] & 2u) && lo[(size_t)c] <= hi[(size_t)c];
     if (floats && !m->has_int_cols) {
+        m->col_repeat.resize((size_t)C);
+        CUDA_TRY(cudaMemcpy(m->col_repeat.data(), repeat.p, sizeof(float) * C, cudaMemcpyDeviceToHost));
         m->col_stream.resize((size_t)C);
         long long any = 0, groups = 0, all = 0;
         for (long long c = 0; c < C; ++c) {
@@ -913,6 +916,83 @@ long long stream_longest(const DeviceInfo& dev, int dtype, int G, long long ref_
     return (long long)(cap * (double)n_rows / (double)std::max<long long>(ref_rows, 1));
 }
 
+// Whether a grouping's genes take the stream kernel, which of them (`level`: kStreamAny, or kStreamGroups in
+// plans of more than kStreamManyGroups groups). Beside the reference, the bitmaps and the table hold
+// the region; what the kernel loses against the rank kernel is its second pass, over the elements of
+// cells hit more than once. For a gene these grow with
+//   pairs   how many other elements of its group equal an element: its targets' entries x the equal
+//           share of its pairs / the groups that they spread over (exp of the entropy of the target
+//           sizes: equal for targets of one size, less where a few hold most cells)
+//   crowd   entries to a cell of the bitmap, which is short of room beside a long reference
+// while the rank kernel gains where a gene holds each value more than a few times. Rank / stream
+// kernel time over 2,124 combinations (1,500 to 190,000 entries a gene, 70 to endless values,
+// uniform, normal and log-like, 1 to 500 targets, both types): pairs + 2 crowd (crowd only above
+// four of a value) below 0.1 1.04 to 9, 0.3 to 0.6 0.9 to 2.4, 0.8 to 1.2 0.5 to 1.5 (190,000 entries on
+// 4,000 values, 150 targets, before this rule 2.30 against 1.52 ms). Log screens (4,000 genes), by the
+// entries' mean of it: 0.1 (50,000 cells, 500 targets) 1.03, 0.5 (200,000, 500) 1.05, 0.7 (300) 0.99, 1.0 (200) 0.95,
+// 1.5 (110) 0.87.
+// Short genes, whose buckets and barriers cost more here, most so for doubles: at 1,100 / 2,000 / 3,000 / 7,000
+// entries float32 log values 0.94 / 0.97 / 1.17 / 1.27 (90 targets), double 0.77 / 0.82 / 0.98 / 1.11, and 0.87 /
+// 0.88 / 1.01 / 0.97 at 300 targets, 1.20 at 15,000.
+constexpr double kStreamRepeats = 0.6;
+struct StreamRule {
+    const hpdex_matrix* m;
+    uint8_t level;
+    bool ties;
+    double targets = 0.0, ref = 0.0, spread = 1.0;  // shares of the rows; groups as above
+    long long n_targets, longest;
+    double room;                                    // bytes for reference, bitmaps and table
+    double key;
+
+    StreamRule(const hpdex_matrix* matrix, const std::vector<long long>& group_rows, int layout_g, bool tie_correction,
+               uint8_t stream_level)
+        : m(matrix), level(stream_level), ties(tie_correction), n_targets((long long)group_rows.size() - 1),
+          longest(stream_longest(m->dev, m->dtype, layout_g, group_rows[0], m->n_rows)), key((double)dtype_size(m->dtype)) {
+        const size_t budget = std::min(m->dev.smem_per_sm - m->dev.smem_reserved, m->dev.smem_optin) - 2048;
+        room = (double)budget - (double)(stream_acc_bytes(layout_g) + stream_bucket_bytes(13));
+        double sum = 0.0, entropy = 0.0;
+        for (size_t g = 1; g < group_rows.size(); ++g) sum += (double)group_rows[g];
+        for (size_t g = 1; g < group_rows.size(); ++g)
+            if (group_rows[g] > 0) entropy -= (double)group_rows[g] / sum * std::log((double)group_rows[g] / sum);
+        const double rows = (double)std::max<long long>(m->n_rows, 1);
+        targets = sum / rows;
+        ref = (double)group_rows[0] / rows;
+        spread = std::exp(entropy);
+    }
+    // a gene of fewer entries is not counted for the stream kernel (kStreamAny: not taken either)
+    long long least(size_t c) const {
+        const bool repeats = m->col_repeat[c] > 1.0f / 20000.0f;
+        if (m->dtype == HPDEX_FLOAT64) return n_targets > 100 ? 12000 : repeats ? 6000 : n_targets > 20 ? 4500 : 3000;
+        return level == kStreamGroups ? kStreamMinEntries : repeats || n_targets > 20 ? 2500 : 1500;
+    }
+    bool takes(size_t c) const {
+        const long long n = m->col_nnz[c];
+        return m->col_stream[c] && m->col_stream[c] <= level && n <= longest && (level == kStreamGroups || n >= least(c));
+    }
+    double repeats(size_t c) const {
+        if (!ties) return 0.0;  // (no second pass)
+        const double n = (double)m->col_nnz[c], t = n * targets, p = (double)m->col_repeat[c];
+        const double space = std::max(room - n * ref * (key + 2.0), 1024.0);
+        const double cells = 8.0 * std::min(space / 2.0, std::max(8.0 * t, t * t / 4.0) + 16.0);
+        return t * p / spread + (n * p > 4.0 ? 2.0 * t / cells : 0.0);
+    }
+    bool pays() const {
+        if (m->col_stream.empty() || longest <= 0) return false;
+        long long all = 0, held = 0, rest_longest = 0;  // (held: entries of the genes long enough)
+        double taken = 0.0, work = 0.0;
+        for (size_t c = 0; c < m->col_nnz.size(); ++c) {
+            const long long n = m->col_nnz[c];
+            all += n;
+            if (!takes(c)) { rest_longest = std::max(rest_longest, n); continue; }
+            if (n >= least(c)) held += n;
+            taken += (double)n;
+            work += (double)n * repeats(c);
+        }
+        return held > 0 && held * 100 >= all * kStreamMinPercent && work <= kStreamRepeats * taken &&
+               (level == kStreamAny || rest_longest * kStreamRestShare * m->dev.sms <= all);
+    }
+};
+
 // The histogram kernel's shared memory: kHistCTAs to an SM, fewer where 64 values of every group
 // need more, down to one; 0 when not even 8 values of every group fit (or the group ids are 32-bit).
 // Its CTAs are slower with a gene than the rank kernel's (384 threads to 1,024; a gene's groups
@@ -993,7 +1073,7 @@ int configure_rank(hpdex_plan* p) {
     return HPDEX_OK;
 }
 
-// Divides a plan's genes (`order`, longest first) between the stream kernel and the rank kernel.
+// A matrix's genes, longest first.
 std::vector<int32_t> longest_first(const hpdex_matrix* m) {
     std::vector<int32_t> order((size_t)m->n_cols);
     std::iota(order.begin(), order.end(), 0);
@@ -1002,26 +1082,17 @@ std::vector<int32_t> longest_first(const hpdex_matrix* m) {
     });
     return order;
 }
+// Divides a plan's genes (`order`, longest first) between the stream kernel and the rank kernel.
 int stream_genes(hpdex_plan* p, const std::vector<int32_t>& order) {
     const hpdex_matrix* m = p->m;
     p->n_stream = 0;
     if (p->stream_mode == 0 || (p->stream_mode < 0 && m->col_stream.empty())) return HPDEX_OK;
-    const long long longest = stream_longest(m->dev, m->dtype, (int)p->G, p->group_rows[0], m->n_rows);
     std::vector<int32_t> mine, rest;
     auto divide = [&](uint8_t level) {  // whether it pays
-        mine.clear();
-        rest.clear();
-        long long all = 0, held = 0, rest_longest = 0;  // (held: entries of the stream kernel's long genes)
-        for (const int32_t c : order) {
-            const long long n = m->col_nnz[(size_t)c];
-            const bool fits = m->col_stream[(size_t)c] && m->col_stream[(size_t)c] <= level && n <= longest;
-            (fits ? mine : rest).push_back(c);
-            all += n;
-            if (!fits) rest_longest = std::max(rest_longest, n);
-            else if (n >= kStreamMinEntries) held += n;
-        }
-        return held > 0 && held * 100 >= all * kStreamMinPercent &&
-               (level == kStreamAny || rest_longest * kStreamRestShare * m->dev.sms <= all);
+        const StreamRule rule(m, p->group_rows, (int)p->G, p->opt.tie_correction != 0, level);
+        if (!rule.pays()) return false;
+        for (const int32_t c : order) (rule.takes((size_t)c) ? mine : rest).push_back(c);
+        return true;
     };
     if (p->stream_mode == 1) mine = order;
     else if (!(p->G > kStreamManyGroups && divide(kStreamGroups)) && !divide(kStreamAny)) return HPDEX_OK;
@@ -2617,6 +2688,13 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
         if (S->mats[(size_t)q->matrix]->has_int_cols) int_genes += S->mats[(size_t)q->matrix]->n_cols;
     const size_t hist_smem = hist_layout(S->dev, GL, int_genes, r, &ha);
     const size_t stream_smem = stream_layout(S->dev, dtype, GL, r, &sa);
+    std::vector<std::unique_ptr<StreamRule>> stream(b.q.size());  // of the queries that take the stream kernel
+    for (size_t i = 0; i < b.q.size() && stream_smem; ++i) {
+        const hpdex_matrix* m = S->mats[(size_t)b.q[i]->matrix];
+        if (!m->stream_any) continue;
+        stream[i].reset(new StreamRule(m, b.q[i]->group_rows, GL, b.q[i]->opt.tie_correction != 0, kStreamAny));
+        if (!stream[i]->pays()) stream[i].reset();
+    }
     std::vector<int32_t> order[3];
     std::vector<uint16_t> order_task[3];
     auto put = [&](int list, int32_t c, size_t i) {
@@ -2630,11 +2708,9 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
             const auto& seg = S->mat_class_start[(size_t)b.q[i]->matrix];
             const int64_t lo = seg[(size_t)(2 * k)], hi = seg[(size_t)(2 * k + 1)];
             const bool hist = hist_smem && m->has_int_cols;
-            const long long longest = stream_smem && m->stream_any
-                ? stream_longest(S->dev, dtype, GL, b.q[i]->group_rows[0], m->n_rows) : -1;
             for (int64_t j = lo; j < hi; ++j) {
                 const int32_t c = ord[(size_t)j];
-                put(hist ? 0 : m->col_nnz[(size_t)c] <= longest && m->col_stream[(size_t)c] == kStreamAny ? 1 : 2, c, i);
+                put(hist ? 0 : stream[i] && stream[i]->takes((size_t)c) ? 1 : 2, c, i);
             }
         }
     const size_t n_hist = order[0].size(), n_stream = order[1].size(), n_rank = order[2].size();

@@ -187,24 +187,28 @@ __device__ __forceinline__ bool pair_count(const PairTable& t, K key, uint32_t g
 }
 
 // Whether a column's values repeat: of kTieSample entries, evenly spaced over it, more than one in
-// eight equal an earlier one (a screen's columns: one in three and more; values drawn from 3,000
-// normal steps: one in nine, where the two kernels take the same time). Sets bit 2 of flags[c] for
-// the columns of at least 2 * kTieSample entries, one block each, and bit 3 where more than five
-// in eight do (plans of many groups take columns below that).
+// eight equal an earlier one. Sets bit 2 of flags[c] for the columns of at least 2 * kTieSample entries, one
+// block each, and bit 3 where more than five in eight do; repeat[c] is the share of the sample's pairs
+// that are equal (an estimate of the sum of squared frequencies of the column's values; 0 for the
+// columns not sampled). The plan decides by both (StreamRule).
 constexpr int kTieSample = 512;
 template <class V>
-__global__ void __launch_bounds__(128) column_ties_kernel(const V* data, const int64_t* indptr, uint32_t* flags) {
+__global__ void __launch_bounds__(128) column_ties_kernel(const V* data, const int64_t* indptr, uint32_t* flags,
+                                                          float* repeat) {
     using K = typename Val<V>::Key;
     __shared__ unsigned long long slot[2 * kTieSample];  // key + 1 (0: empty)
-    __shared__ uint32_t equal;
+    __shared__ uint32_t more[2 * kTieSample];            // elements of the slot's value after its first
+    __shared__ uint32_t equal, pairs, used;
     const long long b = indptr[blockIdx.x], n = indptr[blockIdx.x + 1] - b;
+    if (threadIdx.x == 0) repeat[blockIdx.x] = 0.0f;
     if (n < 2 * kTieSample) return;
-    for (int i = threadIdx.x; i < 2 * kTieSample; i += 128) slot[i] = 0ull;
-    if (threadIdx.x == 0) equal = 0u;
+    for (int i = threadIdx.x; i < 2 * kTieSample; i += 128) { slot[i] = 0ull; more[i] = 0u; }
+    if (threadIdx.x == 0) { equal = 0u; pairs = 0u; used = 0u; }
     __syncthreads();
     for (int i = threadIdx.x; i < kTieSample; i += 128) {
         const V v = data[b + (long long)i * n / kTieSample];
         if (!Val<V>::finite(v) || Val<V>::zero(v)) continue;
+        atomicAdd(&used, 1u);
         const unsigned long long k = (unsigned long long)Val<V>::key(v) + 1ull;
         uint32_t p = pair_hash((unsigned long long)k, 0u) >> 22;  // 1,024 slots, at most half taken
         for (;; p = (p + 1u) & (2u * kTieSample - 1u)) {
@@ -212,12 +216,16 @@ __global__ void __launch_bounds__(128) column_ties_kernel(const V* data, const i
             if (old == 0ull) break;
             if (old == k) {
                 atomicAdd(&equal, 1u);
+                atomicAdd(&pairs, atomicAdd(&more[p], 1u) + 1u);
                 break;
             }
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0 && equal > kTieSample / 8) flags[blockIdx.x] |= equal > 5 * kTieSample / 8 ? 12u : 4u;
+    if (threadIdx.x == 0) {
+        if (equal > kTieSample / 8) flags[blockIdx.x] |= equal > 5 * kTieSample / 8 ? 12u : 4u;
+        if (used > 1u) repeat[blockIdx.x] = 2.0f * (float)pairs / ((float)used * (float)(used - 1u));
+    }
 }
 
 // One 1,024-thread CTA per SM takes genes from the work queue. Per gene:
