@@ -424,13 +424,17 @@ struct hpdex_matrix {
     std::vector<long long> col_nnz;  // host copy for scheduling
     long long max_col_nnz = 0;
     // resident float matrices: which columns may take the stream kernel (kStreamAny, kStreamGroups;
-    // empty: too few), and whether those of kStreamAny hold nearly all entries
+    // empty: too few), and whether those of kStreamAny hold nearly all entries (of the other
+    // than integer columns)
     std::vector<uint8_t> col_stream;
     std::vector<float> col_repeat;   // with col_stream: how far each column repeats its values
                                      // (column_ties_kernel)
     bool stream_any = false;
-    bool has_int_cols = true;  // some column stores only small integers (launches then use the
+    bool has_int_cols = true;  // some column stores only small integers (histogram kernel, or the
                                // rank kernel with the histogram path)
+    std::vector<uint8_t> col_int;  // which, for float matrices that have some (integer types: all)
+    long long n_int_cols = 0;
+    bool int_col(size_t c) const { return has_int_cols && (col_int.empty() || col_int[c]); }
     DeviceInfo dev;
 };
 
@@ -445,11 +449,13 @@ struct hpdex_plan {
     DevBuf<int32_t> order;
     DevBuf<int32_t> queue;       // work counters: rank kernel, stream kernel, genes left, histogram
                                  // kernel
-    DevBuf<int32_t> queue_init;  // their values before a batched run with the stream kernel
-    DevBuf<int32_t> order_stream;  // the stream kernel's genes (n_stream; 0: not used)
-    DevBuf<int32_t> left;        // the rank kernel's genes then: its own, and those the stream
-                                 // kernel leaves
-    int n_stream = 0;
+    DevBuf<int32_t> queue_init;  // their values before a batched run that has genes in `left`
+    // a batched run's genes: of the histogram kernel and of the stream kernel (null: p->order, all of
+    // them), and the rank kernel's, with room for those that the others leave (divide_genes)
+    std::vector<int32_t> longest_first;  // empty: not divided (the one-shot call's chunks)
+    DevBuf<int32_t> order_hist, order_stream, left;
+    int n_hist = 0, n_stream = 0, n_rest = 0;
+    bool rest_histogram = false;  // the rank kernel with the histogram path takes the rest
     int stream_mode = -1;        // hpdex_plan_set_stream
     DevBuf<unsigned long long> err;
     DevBuf<double> U1, P;
@@ -463,10 +469,10 @@ struct hpdex_plan {
     DevBuf<unsigned char> acc;
     DevBuf<uint32_t> cnt;
     RankArgs ra{};
-    StreamArgs sa{};             // stream kernel of the batched form (use_stream)
-    HistArgs ha{};               // histogram kernel of the batched form (use_hist)
-    size_t hist_smem = 0;        // 0: the layout leaves no room for it
-    size_t stream_smem = 0;      // 0: the layout leaves no room for it
+    StreamArgs sa{};             // stream kernel of the batched form (n_stream > 0)
+    HistArgs ha{};               // histogram kernel of the batched form (n_hist > 0)
+    size_t hist_smem = 0;        // 0: off, or the layout leaves no room for it
+    size_t stream_smem = 0;
     bool hist_on = true;         // histogram path allowed (hpdex_plan_set_histogram)
     int nbl = 13;                // bucket table of 2^nbl entries (hpdex_plan_set_bucket_bits)
     int cnt_mode = -1;           // run counters: -1 automatic, 1 shared, 0 global memory
@@ -654,9 +660,22 @@ int matrix_int_hint(hpdex_matrix* m) {
     CUDA_TRY(cudaMemcpy(f.data(), m->col_has_zero.p, sizeof(uint32_t) * C, cudaMemcpyDeviceToHost));
     CUDA_TRY(cudaMemcpy(lo.data(), m->col_kmin.p, sizeof(unsigned long long) * C, cudaMemcpyDeviceToHost));
     CUDA_TRY(cudaMemcpy(hi.data(), m->col_kmax.p, sizeof(unsigned long long) * C, cudaMemcpyDeviceToHost));
-    for (long long c = 0; c < C && !m->has_int_cols; ++c)
-        m->has_int_cols = !(f[(size_t)c] & 2u) && lo[(size_t)c] <= hi[(size_t)c];
-    if (floats && !m->has_int_cols) {
+    auto small_ints = [&](size_t c) { return !(f[c] & 2u) && lo[c] <= hi[c]; };
+    for (long long c = 0; c < C && !m->has_int_cols; ++c) m->has_int_cols = small_ints((size_t)c);
+    if (!floats) {
+        m->n_int_cols = m->has_int_cols ? C : 0;
+    } else {
+        if (m->has_int_cols) {
+            long long ints = 0, others = 0;  // (columns without a nonzero value go with the more)
+            for (long long c = 0; c < C; ++c)
+                if (lo[(size_t)c] <= hi[(size_t)c]) ++(small_ints((size_t)c) ? ints : others);
+            m->col_int.resize((size_t)C);
+            for (long long c = 0; c < C; ++c) {
+                const bool empty = lo[(size_t)c] > hi[(size_t)c];
+                m->col_int[(size_t)c] = empty ? ints > others : small_ints((size_t)c);
+                m->n_int_cols += m->col_int[(size_t)c];
+            }
+        }
         m->col_repeat.resize((size_t)C);
         CUDA_TRY(cudaMemcpy(m->col_repeat.data(), repeat.p, sizeof(float) * C, cudaMemcpyDeviceToHost));
         m->col_stream.resize((size_t)C);
@@ -664,6 +683,7 @@ int matrix_int_hint(hpdex_matrix* m) {
         for (long long c = 0; c < C; ++c) {
             const long long n = m->col_nnz[(size_t)c];
             const bool is_long = n >= kStreamMinEntries;
+            if (m->int_col((size_t)c)) continue;
             m->col_stream[(size_t)c] = (f[(size_t)c] & 8u) ? 0 : is_long && !(f[(size_t)c] & 4u) ? kStreamAny : kStreamGroups;
             all += n;
             if (m->col_stream[(size_t)c] == kStreamAny) any += n;
@@ -982,6 +1002,7 @@ struct StreamRule {
         double taken = 0.0, work = 0.0;
         for (size_t c = 0; c < m->col_nnz.size(); ++c) {
             const long long n = m->col_nnz[c];
+            if (m->int_col(c)) continue;
             all += n;
             if (!takes(c)) { rest_longest = std::max(rest_longest, n); continue; }
             if (n >= least(c)) held += n;
@@ -1012,6 +1033,96 @@ size_t hist_layout(const DeviceInfo& dev, int G, long long genes, const RankLayo
         return acc + 4 * (size_t)a->words;
     }
     return 0;
+}
+
+// A matrix's genes, longest first.
+std::vector<int32_t> longest_first(const hpdex_matrix* m) {
+    std::vector<int32_t> order((size_t)m->n_cols);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
+        return m->col_nnz[(size_t)a] > m->col_nnz[(size_t)b];
+    });
+    return order;
+}
+
+// Whether a rank kernel launch of `ints` entries of integer genes and `floats` of others takes the variant
+// with the histogram path. It costs the others 12% and is worth two or three times the bucket path to
+// integer genes; behind a histogram kernel (of `taken` entries), which leaves few, only where there are
+// hardly any others.
+bool with_histogram(long long ints, long long floats, long long taken) {
+    return taken > 0 ? floats * 8 <= taken : ints > 0 && ints * 16 >= floats;
+}
+
+// Divides a plan's genes, each kernel's longest first: integer genes to the histogram kernel, float genes by
+// StreamRule to the stream kernel, the others to the rank kernel behind them.
+int divide_genes(hpdex_plan* p, const RankLayout& r) {
+    const hpdex_matrix* m = p->m;
+    const int G = (int)p->G;
+    const std::vector<int32_t>& order = p->longest_first;
+    p->n_hist = p->n_stream = p->n_rest = 0;
+    if (order.empty()) return HPDEX_OK;
+    p->stream_smem = p->stream_mode != 0 ? stream_layout(m->dev, m->dtype, G, r, &p->sa) : 0;
+    const bool all_stream = p->stream_smem && p->stream_mode == 1;
+    std::unique_ptr<StreamRule> rule;
+    for (const uint8_t level : {kStreamGroups, kStreamAny}) {
+        if (!p->stream_smem || all_stream || rule || (level == kStreamGroups && p->G <= kStreamManyGroups)) continue;
+        rule.reset(new StreamRule(m, p->group_rows, G, p->opt.tie_correction != 0, level));
+        if (!rule->pays()) rule.reset();
+    }
+    const bool histogram = p->hist_on && m->has_int_cols;
+    p->hist_smem = histogram && !all_stream ? hist_layout(m->dev, G, m->n_int_cols, r, &p->ha) : 0;
+    std::vector<int32_t> hist, stream, rest;
+    long long taken = 0, rest_ints = 0, rest_floats = 0;  // entries
+    for (const int32_t c : order) {
+        const long long n = m->col_nnz[(size_t)c];
+        if (p->hist_smem && m->int_col((size_t)c)) {
+            hist.push_back(c);
+            taken += n;
+        } else if (all_stream || (rule && rule->takes((size_t)c))) {
+            stream.push_back(c);
+        } else {
+            rest.push_back(c);
+            (m->int_col((size_t)c) ? rest_ints : rest_floats) += n;
+        }
+    }
+    p->rest_histogram = histogram && with_histogram(rest_ints, rest_floats, taken);
+    if (hist.empty() && stream.empty()) return HPDEX_OK;  // the rank kernel takes p->order
+
+    auto upload = [&](DevBuf<int32_t>& d, const std::vector<int32_t>& genes) -> int {
+        TRY(d.alloc(genes.size() == order.size() ? 0 : genes.size()));
+        if (d.p) CUDA_TRY(cudaMemcpy(d.p, genes.data(), sizeof(int32_t) * genes.size(), cudaMemcpyHostToDevice));
+        return HPDEX_OK;
+    };
+    TRY(upload(p->order_hist, hist));
+    TRY(upload(p->order_stream, stream));
+    TRY(p->left.alloc(order.size()));
+    TRY(p->queue_init.alloc(rest.empty() ? 0 : 4));
+    if (!rest.empty()) {
+        const int32_t init[4] = {0, 0, (int32_t)rest.size(), 0};
+        CUDA_TRY(cudaMemcpy(p->left.p, rest.data(), sizeof(int32_t) * rest.size(), cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpy(p->queue_init.p, init, sizeof init, cudaMemcpyHostToDevice));
+    }
+    HistArgs& h = p->ha;
+    h.tasks = p->d_task.p;
+    h.order = p->order_hist.p ? p->order_hist.p : p->order.p;
+    h.n_order = (int32_t)hist.size();
+    h.queue = p->queue.p + 3;
+    h.n_left = p->queue.p + 2;
+    h.left = p->left.p;
+    StreamArgs& sa = p->sa;
+    sa.tasks = p->d_task.p;
+    sa.order = p->order_stream.p ? p->order_stream.p : p->order.p;
+    sa.n_order = (int32_t)stream.size();
+    sa.queue = p->queue.p + 1;
+    sa.n_left = p->queue.p + 2;
+    sa.left = p->left.p;
+    sa.dk_global = p->dk.p;
+    sa.dg_global = p->dg.p;
+    sa.slice = r.slice;
+    p->n_hist = (int)hist.size();
+    p->n_stream = (int)stream.size();
+    p->n_rest = (int)rest.size();
+    return HPDEX_OK;
 }
 
 int configure_rank(hpdex_plan* p) {
@@ -1046,74 +1157,8 @@ int configure_rank(hpdex_plan* p) {
     a.any_compact = t.compact_decode;
     set_layout_args(a, r, G, p->dk.p, p->dg.p, p->ek.p, p->eg.p, p->acc.p, p->cnt.p);
 
-    p->hist_smem = m->has_int_cols ? hist_layout(m->dev, G, m->n_cols, r, &p->ha) : 0;
-    if (p->hist_smem) {
-        TRY(p->left.alloc(std::max<long long>(m->n_cols, 1)));
-        HistArgs& h = p->ha;
-        h.tasks = p->d_task.p;
-        h.order = p->order.p;
-        h.n_order = (int32_t)m->n_cols;
-        h.queue = p->queue.p + 3;
-        h.n_left = p->queue.p + 2;
-        h.left = p->left.p;
-    }
-    p->stream_smem = p->n_stream ? stream_layout(m->dev, m->dtype, G, r, &p->sa) : 0;
-    if (p->stream_smem) {
-        StreamArgs& sa = p->sa;
-        sa.tasks = p->d_task.p;
-        sa.order = p->order_stream.p ? p->order_stream.p : p->order.p;
-        sa.n_order = p->n_stream;
-        sa.queue = p->queue.p + 1;
-        sa.n_left = p->queue.p + 2;
-        sa.left = p->left.p;
-        sa.dk_global = p->dk.p;
-        sa.dg_global = p->dg.p;
-        sa.slice = r.slice;
-    }
-    return HPDEX_OK;
+    return divide_genes(p, r);
 }
-
-// A matrix's genes, longest first.
-std::vector<int32_t> longest_first(const hpdex_matrix* m) {
-    std::vector<int32_t> order((size_t)m->n_cols);
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
-        return m->col_nnz[(size_t)a] > m->col_nnz[(size_t)b];
-    });
-    return order;
-}
-// Divides a plan's genes (`order`, longest first) between the stream kernel and the rank kernel.
-int stream_genes(hpdex_plan* p, const std::vector<int32_t>& order) {
-    const hpdex_matrix* m = p->m;
-    p->n_stream = 0;
-    if (p->stream_mode == 0 || (p->stream_mode < 0 && m->col_stream.empty())) return HPDEX_OK;
-    std::vector<int32_t> mine, rest;
-    auto divide = [&](uint8_t level) {  // whether it pays
-        const StreamRule rule(m, p->group_rows, (int)p->G, p->opt.tie_correction != 0, level);
-        if (!rule.pays()) return false;
-        for (const int32_t c : order) (rule.takes((size_t)c) ? mine : rest).push_back(c);
-        return true;
-    };
-    if (p->stream_mode == 1) mine = order;
-    else if (!(p->G > kStreamManyGroups && divide(kStreamGroups)) && !divide(kStreamAny)) return HPDEX_OK;
-    if (mine.empty()) return HPDEX_OK;
-    const int32_t init[4] = {0, 0, (int32_t)rest.size(), 0};
-    TRY(p->left.alloc(order.size()));
-    TRY(p->order_stream.alloc(rest.empty() ? 0 : mine.size()));  // (all genes: p->order)
-    TRY(p->queue_init.alloc(rest.empty() ? 0 : 4));
-    if (!rest.empty()) {
-        CUDA_TRY(cudaMemcpy(p->order_stream.p, mine.data(), sizeof(int32_t) * mine.size(), cudaMemcpyHostToDevice));
-        CUDA_TRY(cudaMemcpy(p->left.p, rest.data(), sizeof(int32_t) * rest.size(), cudaMemcpyHostToDevice));
-        CUDA_TRY(cudaMemcpy(p->queue_init.p, init, sizeof init, cudaMemcpyHostToDevice));
-    }
-    p->n_stream = (int)mine.size();
-    return HPDEX_OK;
-}
-
-// The stream kernel is off while a matrix holds integer columns (histogram path); the histogram
-// kernel takes those.
-bool use_hist(const hpdex_plan* p) { return p->hist_smem != 0 && !p->ra.no_histogram; }
-bool use_stream(const hpdex_plan* p) { return p->stream_smem != 0 && p->ra.no_histogram; }
 
 int launch_pvalues_asymptotic(hpdex_plan* p, cudaStream_t s) {
     PArgs a{};
@@ -1339,29 +1384,29 @@ int enqueue_rank(hpdex_plan* p, int mode, cudaStream_t s, int* launches) {
     if (mode == HPDEX_MODE_BATCHED) {
         p->ra.single_gene = -1;
         RankArgs a = p->ra;
-        if (use_hist(p)) {
+        a.no_histogram = p->rest_histogram ? 0 : 1;
+        // (the counters of all kernels; the rank kernel's genes start with those already in `left`)
+        if (p->n_rest > 0 && (p->n_hist || p->n_stream))
+            CUDA_TRY(cudaMemcpyAsync(p->queue.p, p->queue_init.p, 4 * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
+        else
             CUDA_TRY(cudaMemsetAsync(p->queue.p, 0, 4 * sizeof(int32_t), s));
+        if (p->n_hist) {
             HistArgs h = p->ha;
             h.erfc_table = a.erfc_table;
             TRY(rank_status(hist_launch(p->m->dtype, h, p->m->dev.sms, p->hist_smem, s), "histogram kernel launch"));
             *launches += 1;
-            a.order = p->left.p;
-            a.n_order_dev = h.n_left;
-        } else if (!use_stream(p)) {
-            CUDA_TRY(cudaMemsetAsync(p->queue.p, 0, sizeof(int32_t), s));
-        } else {  // the rank kernel then takes its own genes and those the stream kernel left
-            if (p->queue_init.p)
-                CUDA_TRY(cudaMemcpyAsync(p->queue.p, p->queue_init.p, 4 * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
-            else
-                CUDA_TRY(cudaMemsetAsync(p->queue.p, 0, 4 * sizeof(int32_t), s));
+        }
+        if (p->n_stream) {
             StreamArgs sa = p->sa;
             sa.erfc_table = a.erfc_table;
             auto launch = p->m->dtype == HPDEX_FLOAT32 ? stream_launch_f32 : stream_launch_f64;
             const int grid = std::min(p->m->dev.sms, p->n_stream);
             TRY(rank_status(launch(sa, grid, p->stream_smem, s), "stream kernel launch"));
             *launches += 1;
+        }
+        if (p->n_hist || p->n_stream) {  // its own genes and those the others left
             a.order = p->left.p;
-            a.n_order_dev = sa.n_left;
+            a.n_order_dev = p->queue.p + 2;
         }
         TRY(rank_status(rank_launch(p->m->dtype, a, p->rank_grid, p->rank_smem, s), "rank kernel launch"));
         *launches += 1;
@@ -1765,9 +1810,8 @@ int plan_create(hpdex_matrix* m, const int32_t* group_id, int64_t n_targets,
     // longest genes first: the work queue hands them out before the short tail
     TRY(p->order.alloc(std::max<long long>(C, 1)));
     if (lpt_order && C) {
-        const std::vector<int32_t> order = longest_first(m);
-        CUDA_TRY(cudaMemcpy(p->order.p, order.data(), sizeof(int32_t) * C, cudaMemcpyHostToDevice));
-        TRY(stream_genes(p.get(), order));
+        p->longest_first = longest_first(m);
+        CUDA_TRY(cudaMemcpy(p->order.p, p->longest_first.data(), sizeof(int32_t) * C, cudaMemcpyHostToDevice));
     }
     TRY(p->queue.alloc(4));
     TRY(p->err.alloc(kErrWords));
@@ -1827,7 +1871,7 @@ int hpdex_plan_run(hpdex_plan* p, int32_t mode) {
             CUDA_TRY(cudaGraphInstantiate(&p->graph_exec, g, 0));
         }
         CUDA_TRY(cudaGraphLaunch(p->graph_exec, s));
-        launches = (p->m->n_cols > 0 ? (use_stream(p) || use_hist(p) ? 3 : 2) : 0) + (!p->fused_pvalues && p->T * p->m->n_cols > 0 ? 1 : 0);
+        launches = (p->m->n_cols > 0 ? 2 + (p->n_hist > 0) + (p->n_stream > 0) : 0) + (!p->fused_pvalues && p->T * p->m->n_cols > 0 ? 1 : 0);
     } else {
         CUDA_TRY(cudaEventRecord(p->ev[0], s));
         CUDA_TRY(cudaMemsetAsync(p->err.p, 0xff, kErrWords * sizeof(unsigned long long), s));
@@ -1849,6 +1893,19 @@ int hpdex_plan_run(hpdex_plan* p, int32_t mode) {
     CUDA_TRY(cudaEventElapsedTime(&p->last_ms[2], p->ev[1], p->ev[2]));
     return check_device_errors(p);
 }
+
+namespace {
+// The plan's kernels and their genes after a switch; the other launch settings stay as they were.
+int divide_again(hpdex_plan* p) {
+    const RankArgs keep = p->ra;
+    const int st = configure_rank(p);
+    p->ra.erfc_table = keep.erfc_table;
+    p->ra.drain_wait = keep.drain_wait;
+    if (p->graph_exec) { cudaGraphExecDestroy(p->graph_exec); p->graph_exec = nullptr; }  // re-captured
+    if (p->graph) { cudaGraphDestroy(p->graph); p->graph = nullptr; }
+    return st;
+}
+}  // namespace
 
 int hpdex_plan_autotune(hpdex_plan* p, int32_t reps, int32_t* run_counters_out,
                         int32_t* bucket_bits_out, float* ms_out) {
@@ -1952,29 +2009,17 @@ int hpdex_plan_set_run_counters(hpdex_plan* p, int32_t mode) {
 
 int hpdex_plan_set_histogram(hpdex_plan* p, int32_t on) {
     if (!p) return fail(HPDEX_ERR_ARGUMENT, "plan is NULL");
+    if (p->hist_on == (on != 0)) return HPDEX_OK;
     p->hist_on = on != 0;
-    const int32_t off = (p->hist_on && p->m->has_int_cols) ? 0 : 1;
-    if (p->ra.no_histogram == off) return HPDEX_OK;
-    p->ra.no_histogram = off;
-    if (p->graph_exec) { cudaGraphExecDestroy(p->graph_exec); p->graph_exec = nullptr; }  // re-captured
-    if (p->graph) { cudaGraphDestroy(p->graph); p->graph = nullptr; }
-    return HPDEX_OK;
+    return divide_again(p);
 }
 
 int hpdex_plan_set_stream(hpdex_plan* p, int32_t mode) {
     if (!p) return fail(HPDEX_ERR_ARGUMENT, "plan is NULL");
     if (mode < -1 || mode > 1) return fail(HPDEX_ERR_ARGUMENT, "stream mode must be -1, 0 or 1");
     if (mode == p->stream_mode) return HPDEX_OK;
-    const RankArgs keep = p->ra;  // the plan's other launch settings stay as they were
     p->stream_mode = mode;
-    int st = stream_genes(p, longest_first(p->m));
-    if (st == HPDEX_OK) st = configure_rank(p);
-    p->ra.erfc_table = keep.erfc_table;
-    p->ra.drain_wait = keep.drain_wait;
-    p->ra.no_histogram = keep.no_histogram;
-    if (p->graph_exec) { cudaGraphExecDestroy(p->graph_exec); p->graph_exec = nullptr; }  // re-captured
-    if (p->graph) { cudaGraphDestroy(p->graph); p->graph = nullptr; }
-    return st;
+    return divide_again(p);
 }
 
 int hpdex_plan_set_drain_wait(hpdex_plan* p, int32_t on) {
@@ -2679,13 +2724,12 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
         t.compact_decode = compact_decode(q->group_rows, R);
     }
     // a work queue per kernel over the (query, gene) items of the batch, longest first by nnz class:
-    // integer matrices to the histogram kernel, long float genes whose values seldom repeat to the
+    // integer genes to the histogram kernel, long float genes whose values seldom repeat to the
     // stream kernel, the others to the rank kernel
     HistArgs ha{};
     StreamArgs sa{};
     long long int_genes = 0;
-    for (ServerQuery* q : b.q)
-        if (S->mats[(size_t)q->matrix]->has_int_cols) int_genes += S->mats[(size_t)q->matrix]->n_cols;
+    for (ServerQuery* q : b.q) int_genes += S->mats[(size_t)q->matrix]->n_int_cols;
     const size_t hist_smem = hist_layout(S->dev, GL, int_genes, r, &ha);
     const size_t stream_smem = stream_layout(S->dev, dtype, GL, r, &sa);
     std::vector<std::unique_ptr<StreamRule>> stream(b.q.size());  // of the queries that take the stream kernel
@@ -2701,16 +2745,19 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
         order[list].push_back(c);
         order_task[list].push_back((uint16_t)i);
     };
+    long long taken = 0, rest_ints = 0, rest_floats = 0;  // entries
     for (int k = 63; k >= 0; --k)
         for (size_t i = 0; i < b.q.size(); ++i) {
             const hpdex_matrix* m = S->mats[(size_t)b.q[i]->matrix];
             const auto& ord = S->mat_order[(size_t)b.q[i]->matrix];
             const auto& seg = S->mat_class_start[(size_t)b.q[i]->matrix];
             const int64_t lo = seg[(size_t)(2 * k)], hi = seg[(size_t)(2 * k + 1)];
-            const bool hist = hist_smem && m->has_int_cols;
             for (int64_t j = lo; j < hi; ++j) {
                 const int32_t c = ord[(size_t)j];
-                put(hist ? 0 : stream[i] && stream[i]->takes((size_t)c) ? 1 : 2, c, i);
+                const bool is_int = m->int_col((size_t)c);
+                const int list = hist_smem && is_int ? 0 : stream[i] && stream[i]->takes((size_t)c) ? 1 : 2;
+                put(list, c, i);
+                if (list != 1) (list == 0 ? taken : is_int ? rest_ints : rest_floats) += m->col_nnz[(size_t)c];
             }
         }
     const size_t n_hist = order[0].size(), n_stream = order[1].size(), n_rank = order[2].size();
@@ -2783,14 +2830,7 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
         a.n_order_dev = b.queue.p + 2;
         a.queue = b.queue.p;
         a.single_gene = -1;
-        // the histogram variant costs float genes 12%: only where the integer genes are this
-        // kernel's, or all that is left for it
-        bool all_int = true, any_int = false;
-        for (auto* q : b.q) {
-            all_int = all_int && S->mats[(size_t)q->matrix]->has_int_cols;
-            any_int = any_int || S->mats[(size_t)q->matrix]->has_int_cols;
-        }
-        a.no_histogram = (n_hist ? all_int : any_int) ? 0 : 1;
+        a.no_histogram = with_histogram(rest_ints, rest_floats, taken) ? 0 : 1;
         for (const RankTask& t : tasks) a.any_compact |= t.compact_decode;
         set_layout_args(a, r, GL, b.dk.p, b.dg.p, b.ek.p, b.eg.p, b.acc.p, b.cnt.p);
         TRY(rank_status(rank_launch(dtype, a, r.grid, r.smem, st), "rank kernel launch"));

@@ -189,8 +189,9 @@ class Plan:
                 "ms": {f"{c}/2^{b}": round(float(t), 4) for (c, b), t in zip(names, ms)}}
 
     def set_stream(self, mode: int) -> None:
-        """Diagnostic: float genes on the stream kernel: long ones whose values seldom repeat (-1,
-        the default), none (0) or all (1); results do not change."""
+        """Diagnostic: genes of a float matrix on the stream kernel: long ones whose values seldom meet
+        in a group, other than integer counts (-1, the default), none (0) or all (1); results do
+        not change."""
         _lib.check(_lib.lib().hpdex_plan_set_stream(self._h, int(mode)))
 
     def set_drain_wait(self, on: bool) -> None:

@@ -246,7 +246,8 @@ int hpdex_plan_autotune(hpdex_plan* p, int32_t reps, int32_t* run_counters_out,
 int hpdex_plan_set_histogram(hpdex_plan* p, int32_t on);
 
 /* Diagnostic: which genes of a batched run take the stream kernel (float matrices): -1 (default) long
- * genes whose values seldom repeat, 0 none, 1 all. Results do not change. */
+ * genes whose values seldom meet in a group, other than integer counts; 0 none; 1 all, integer counts
+ * too. Results do not change. */
 int hpdex_plan_set_stream(hpdex_plan* plan, int32_t mode);
 
 /* Diagnostic. The rank kernel lets a warp resolve a large bucket while other warps of its CTA
