@@ -433,7 +433,7 @@ struct hpdex_matrix {
     bool has_int_cols = true;  // some column stores only small integers (histogram kernel, or the
                                // rank kernel with the histogram path)
     std::vector<uint8_t> col_int;  // which, for float matrices that have some (integer types: all)
-    long long n_int_cols = 0;
+    long long n_int_cols = 0, int_longest = 0, int_entries = 0;  // their count, longest, entries
     bool int_col(size_t c) const { return has_int_cols && (col_int.empty() || col_int[c]); }
     DeviceInfo dev;
 };
@@ -662,9 +662,7 @@ int matrix_int_hint(hpdex_matrix* m) {
     CUDA_TRY(cudaMemcpy(hi.data(), m->col_kmax.p, sizeof(unsigned long long) * C, cudaMemcpyDeviceToHost));
     auto small_ints = [&](size_t c) { return !(f[c] & 2u) && lo[c] <= hi[c]; };
     for (long long c = 0; c < C && !m->has_int_cols; ++c) m->has_int_cols = small_ints((size_t)c);
-    if (!floats) {
-        m->n_int_cols = m->has_int_cols ? C : 0;
-    } else {
+    if (floats) {
         if (m->has_int_cols) {
             long long ints = 0, others = 0;  // (columns without a nonzero value go with the more)
             for (long long c = 0; c < C; ++c)
@@ -673,7 +671,6 @@ int matrix_int_hint(hpdex_matrix* m) {
             for (long long c = 0; c < C; ++c) {
                 const bool empty = lo[(size_t)c] > hi[(size_t)c];
                 m->col_int[(size_t)c] = empty ? ints > others : small_ints((size_t)c);
-                m->n_int_cols += m->col_int[(size_t)c];
             }
         }
         m->col_repeat.resize((size_t)C);
@@ -691,6 +688,12 @@ int matrix_int_hint(hpdex_matrix* m) {
         }
         m->stream_any = any > 0 && any * 100 >= all * kStreamMinPercent;
         if (groups == 0 || groups * 100 < all * kStreamMinPercent) m->col_stream.clear();
+    }
+    for (long long c = 0; c < C; ++c) {
+        if (!m->int_col((size_t)c)) continue;
+        ++m->n_int_cols;
+        m->int_longest = std::max(m->int_longest, m->col_nnz[(size_t)c]);
+        m->int_entries += m->col_nnz[(size_t)c];
     }
     return HPDEX_OK;
 }
@@ -1022,8 +1025,14 @@ struct StreamRule {
 // 16,000 cells 2.3 (50 groups), 1.8 (120), 1.4 (200), 1.2 (332), 0.8 (500); 500 genes 1.3, 0.8,
 // 0.6, 0.8, 0.6; 200 genes 1.0, 0.7, 0.8, 0.6, 0.5; 1,000 genes of 50,000 cells 1.3, 0.9, 0.95, 1.0,
 // 0.8.
-size_t hist_layout(const DeviceInfo& dev, int G, long long genes, const RankLayout& r, HistArgs* a) {
+// Nor where one gene outlasts the others: an entry takes a CTA here 0.45 ns, a gene the rank kernel 10 us and
+// more, so the longest has at most 20,000 entries for each gene that an SM gets, or half an SM's
+// entries. One gene of 200,000 / 400,000 / 1,000,000 entries beside 600 of 2,000: 0.67 / 0.47 / 0.41; beside 4,000
+// of 1,000: 2.4 / 1.4 / 0.63; beside 1,500 of 20,000: 0.97 / 0.62 / 0.38.
+size_t hist_layout(const DeviceInfo& dev, int G, long long genes, long long longest, long long entries, const RankLayout& r,
+                   HistArgs* a) {
     if (!r.acc_in || genes * 16 < (long long)dev.sms * std::max(48, G)) return 0;
+    if (longest * dev.sms > std::max(20000 * genes, entries / 2)) return 0;
     for (int ctas = kHistCTAs; ctas >= 1; --ctas) {
         const size_t room = std::min(dev.smem_per_sm / ctas - dev.smem_reserved, dev.smem_optin) - 2048;
         const size_t acc = hist_acc_bytes(G), values = ctas > 1 ? 64 : 8;
@@ -1070,7 +1079,7 @@ int divide_genes(hpdex_plan* p, const RankLayout& r) {
         if (!rule->pays()) rule.reset();
     }
     const bool histogram = p->hist_on && m->has_int_cols;
-    p->hist_smem = histogram && !all_stream ? hist_layout(m->dev, G, m->n_int_cols, r, &p->ha) : 0;
+    p->hist_smem = histogram && !all_stream ? hist_layout(m->dev, G, m->n_int_cols, m->int_longest, m->int_entries, r, &p->ha) : 0;
     std::vector<int32_t> hist, stream, rest;
     long long taken = 0, rest_ints = 0, rest_floats = 0;  // entries
     for (const int32_t c : order) {
@@ -2728,9 +2737,14 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
     // stream kernel, the others to the rank kernel
     HistArgs ha{};
     StreamArgs sa{};
-    long long int_genes = 0;
-    for (ServerQuery* q : b.q) int_genes += S->mats[(size_t)q->matrix]->n_int_cols;
-    const size_t hist_smem = hist_layout(S->dev, GL, int_genes, r, &ha);
+    long long int_genes = 0, int_longest = 0, int_entries = 0;
+    for (ServerQuery* q : b.q) {
+        const hpdex_matrix* m = S->mats[(size_t)q->matrix];
+        int_genes += m->n_int_cols;
+        int_longest = std::max(int_longest, m->int_longest);
+        int_entries += m->int_entries;
+    }
+    const size_t hist_smem = hist_layout(S->dev, GL, int_genes, int_longest, int_entries, r, &ha);
     const size_t stream_smem = stream_layout(S->dev, dtype, GL, r, &sa);
     std::vector<std::unique_ptr<StreamRule>> stream(b.q.size());  // of the queries that take the stream kernel
     for (size_t i = 0; i < b.q.size() && stream_smem; ++i) {
