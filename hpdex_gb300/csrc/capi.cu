@@ -455,6 +455,7 @@ struct hpdex_plan {
     std::vector<int32_t> longest_first;  // empty: not divided (the one-shot call's chunks)
     DevBuf<int32_t> order_hist, order_stream, left;
     int n_hist = 0, n_stream = 0, n_rest = 0;
+    bool rank_minor = false;      // most entries are the other kernels'
     bool rest_histogram = false;  // the rank kernel with the histogram path takes the rest
     int stream_mode = -1;        // hpdex_plan_set_stream
     DevBuf<unsigned long long> err;
@@ -1069,6 +1070,7 @@ int divide_genes(hpdex_plan* p, const RankLayout& r) {
     const int G = (int)p->G;
     const std::vector<int32_t>& order = p->longest_first;
     p->n_hist = p->n_stream = p->n_rest = 0;
+    p->rank_minor = false;
     if (order.empty()) return HPDEX_OK;
     p->stream_smem = p->stream_mode != 0 ? stream_layout(m->dev, m->dtype, G, r, &p->sa) : 0;
     const bool all_stream = p->stream_smem && p->stream_mode == 1;
@@ -1131,6 +1133,7 @@ int divide_genes(hpdex_plan* p, const RankLayout& r) {
     p->n_hist = (int)hist.size();
     p->n_stream = (int)stream.size();
     p->n_rest = (int)rest.size();
+    p->rank_minor = (rest_ints + rest_floats) * 2 < m->nnz;
     return HPDEX_OK;
 }
 
@@ -1925,6 +1928,10 @@ int hpdex_plan_autotune(hpdex_plan* p, int32_t reps, int32_t* run_counters_out,
     // one untimed run) is kept
     const int32_t modes[2] = {1, 0}, bits[2] = {13, 12};
     const int32_t old_mode = p->cnt_mode, old_bits = p->nbl;
+    // (where the rank kernel gets the smaller part the candidates differ by noise, and the fastest of a
+    // run would be kept for plain runs and the genes left, which it may cost a third: the plan
+    // keeps the layout it has)
+    const bool keep = p->rank_minor;
     float best = 0.0f;
     int32_t best_mode = 1, best_bits = 13;
     int st = HPDEX_OK;
@@ -1952,10 +1959,10 @@ int hpdex_plan_autotune(hpdex_plan* p, int32_t reps, int32_t* run_counters_out,
         hpdex_plan_set_bucket_bits(p, old_bits);
         return fail(st, "%s", msg.c_str());
     }
-    TRY(hpdex_plan_set_run_counters(p, best_mode));
-    TRY(hpdex_plan_set_bucket_bits(p, best_bits));
-    if (run_counters_out) *run_counters_out = best_mode;
-    if (bucket_bits_out) *bucket_bits_out = best_bits;
+    TRY(hpdex_plan_set_run_counters(p, keep ? old_mode : best_mode));
+    TRY(hpdex_plan_set_bucket_bits(p, keep ? old_bits : best_bits));
+    if (run_counters_out) *run_counters_out = !keep ? best_mode : p->ra.cnt_in_smem ? 1 : 0;
+    if (bucket_bits_out) *bucket_bits_out = p->nbl;
     return HPDEX_OK;
 }
 

@@ -178,7 +178,8 @@ class Plan:
     def autotune(self, reps: int = 3) -> dict:
         """Times the plan under each candidate rank-kernel layout (run counters in shared or
         global memory, bucket table of 2^13 or 2^12 entries) and keeps the fastest; results do
-        not change. Returns the choice and the mean time of every candidate."""
+        not change. A plan most of whose entries the histogram or the stream kernel takes keeps the
+        layout it has. Returns the choice and the mean time of every candidate."""
         mode, bits = ctypes.c_int32(), ctypes.c_int32()
         ms = (ctypes.c_float * 4)()
         _lib.check(_lib.lib().hpdex_plan_autotune(self._h, int(reps), ctypes.byref(mode),
