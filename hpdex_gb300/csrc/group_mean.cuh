@@ -6,15 +6,20 @@
 // do not) or by valid[g] (explicit values only); a zero denominator gives 0. Output is
 // flat [gene * G + g] like the reference. One CTA per gene.
 //
-// The sums are exact. A double atomic add in shared memory is a compare-and-swap loop, which
+// A double atomic add in shared memory is a compare-and-swap loop, which
 // on a gene's random groups retries for every lane that shares a word, while a 32-bit integer
 // add is a single native operation. So a gene's values are added as fixed-point integers of 64 or 96 bits
 // (two or three 32-bit words with the carry taken from the returned old value), scaled by a
-// power of two that its key range and entry count choose so that neither the largest sum
-// overflows nor the smallest value loses a bit. Integer sums do not depend on the order of
-// the atomics; one rounding turns them into doubles. A value that would lose a bit (only
-// possible where the smallest magnitude is not known, a gene of both signs) makes the CTA
-// repeat the gene with double atomics.
+// power of two that its key range and entry count choose so that the largest sum does not
+// overflow. Such sums are exact and do not depend on the order of the atomics; one rounding turns
+// them into doubles. They hold every bit of the gene's values unless the lowest bit of some value lies
+// more than 94 bits, less those of the entry count, below the top of the largest (doubles: a
+// value below 2^-25 of the largest in a gene of 100,000 entries; float32: 2^-54). A value that would
+// lose a bit makes the CTA repeat the gene with double atomics, whose sums round once per
+// addition and depend on their order; the same holds for more groups than shared memory has room
+// for. (300 genes of 200,000 float32 values over 30 decades: 1.36 ms, double atomics at once 1.30. A test
+// that ends the first pass at such a value gave 1.11, but cost the genes of three words that
+// lose none up to 9%.)
 #pragma once
 #include <cstdint>
 #include <type_traits>
