@@ -641,48 +641,48 @@ constexpr uint8_t kStreamAny = 1, kStreamGroups = 2;  // values of hpdex_matrix:
 
 // Sets m->has_int_cols from the column flags of the key-range pass: some column with finite
 // nonzero values, all of them small integers (bit 1 of col_has_zero clear).
-// For float data first which columns repeat their values (column_ties_kernel).
+// For float data that holds others, also how the columns repeat their values (column_ties_kernel).
 int matrix_int_hint(hpdex_matrix* m) {
     const long long C = m->n_cols;
     m->has_int_cols = false;
     if (C == 0) return HPDEX_OK;
     const bool floats = m->dtype == HPDEX_FLOAT32 || m->dtype == HPDEX_FLOAT64;
-    DevBuf<float> repeat;
-    if (floats) {
-        TRY(repeat.alloc((size_t)C));
-        if (m->dtype == HPDEX_FLOAT32)
-            column_ties_kernel<float><<<(int)C, 128>>>(reinterpret_cast<const float*>(m->data.p), m->indptr.p, m->col_has_zero.p, repeat.p);
-        else
-            column_ties_kernel<double><<<(int)C, 128>>>(reinterpret_cast<const double*>(m->data.p), m->indptr.p, m->col_has_zero.p, repeat.p);
-        CUDA_TRY(cudaGetLastError());
-    }
     std::vector<uint32_t> f((size_t)C);
     std::vector<unsigned long long> lo((size_t)C), hi((size_t)C);
     CUDA_TRY(cudaMemcpy(f.data(), m->col_has_zero.p, sizeof(uint32_t) * C, cudaMemcpyDeviceToHost));
     CUDA_TRY(cudaMemcpy(lo.data(), m->col_kmin.p, sizeof(unsigned long long) * C, cudaMemcpyDeviceToHost));
     CUDA_TRY(cudaMemcpy(hi.data(), m->col_kmax.p, sizeof(unsigned long long) * C, cudaMemcpyDeviceToHost));
-    auto small_ints = [&](size_t c) { return !(f[c] & 2u) && lo[c] <= hi[c]; };
-    for (long long c = 0; c < C && !m->has_int_cols; ++c) m->has_int_cols = small_ints((size_t)c);
-    if (floats) {
-        if (m->has_int_cols) {
-            long long ints = 0, others = 0;  // (columns without a nonzero value go with the more)
-            for (long long c = 0; c < C; ++c)
-                if (lo[(size_t)c] <= hi[(size_t)c]) ++(small_ints((size_t)c) ? ints : others);
-            m->col_int.resize((size_t)C);
-            for (long long c = 0; c < C; ++c) {
-                const bool empty = lo[(size_t)c] > hi[(size_t)c];
-                m->col_int[(size_t)c] = empty ? ints > others : small_ints((size_t)c);
-            }
-        }
+    auto empty = [&](size_t c) { return lo[c] > hi[c]; };
+    auto small_ints = [&](size_t c) { return !(f[c] & 2u) && !empty(c); };
+    long long ints = 0, others = 0;
+    for (long long c = 0; c < C; ++c)
+        if (!empty((size_t)c)) ++(small_ints((size_t)c) ? ints : others);
+    m->has_int_cols = ints > 0;
+    if (floats && ints > 0 && others > 0) {  // (columns without a nonzero value go with the more)
+        m->col_int.resize((size_t)C);
+        for (long long c = 0; c < C; ++c) m->col_int[(size_t)c] = empty((size_t)c) ? ints > others : small_ints((size_t)c);
+    }
+    if (floats && others > 0) {
+        DevBuf<ColumnTies> d_ties;
+        std::vector<ColumnTies> ties((size_t)C);
+        TRY(d_ties.alloc((size_t)C));
+        if (m->dtype == HPDEX_FLOAT32)
+            column_ties_kernel<float><<<(int)C, 128>>>(reinterpret_cast<const float*>(m->data.p), m->indptr.p, d_ties.p);
+        else
+            column_ties_kernel<double><<<(int)C, 128>>>(reinterpret_cast<const double*>(m->data.p), m->indptr.p, d_ties.p);
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaMemcpy(ties.data(), d_ties.p, sizeof(ColumnTies) * C, cudaMemcpyDeviceToHost));
         m->col_repeat.resize((size_t)C);
-        CUDA_TRY(cudaMemcpy(m->col_repeat.data(), repeat.p, sizeof(float) * C, cudaMemcpyDeviceToHost));
         m->col_stream.resize((size_t)C);
         long long any = 0, groups = 0, all = 0;
         for (long long c = 0; c < C; ++c) {
             const long long n = m->col_nnz[(size_t)c];
             const bool is_long = n >= kStreamMinEntries;
             if (m->int_col((size_t)c)) continue;
-            m->col_stream[(size_t)c] = (f[(size_t)c] & 8u) ? 0 : is_long && !(f[(size_t)c] & 4u) ? kStreamAny : kStreamGroups;
+            const ColumnTies& t = ties[(size_t)c];
+            m->col_repeat[(size_t)c] = t.repeat;
+            m->col_stream[(size_t)c] = t.equal > 5 * kTieSample / 8 ? 0
+                                       : is_long && t.equal <= kTieSample / 8 ? kStreamAny : kStreamGroups;
             all += n;
             if (m->col_stream[(size_t)c] == kStreamAny) any += n;
             if (m->col_stream[(size_t)c] && is_long) groups += n;

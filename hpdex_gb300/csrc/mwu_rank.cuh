@@ -67,9 +67,7 @@ struct RankTask {
     const unsigned long long* col_kmax;  //   (kmin > kmax: none)
     const uint32_t* col_has_zero;        // per column: bit 0 stores an explicit finite zero,
                                          // bit 1 stores a finite value that is not an integer
-                                         // of magnitude below 2^31 (no histogram path), bit 2
-                                         // repeats its values, bit 3 most of them
-                                         // (column_ties_kernel)
+                                         // of magnitude below 2^31 (no histogram path)
     int64_t n_rows;
     int32_t n_cols;
     int32_t G;                 // n_targets + 1 (at most the launch's layout G)

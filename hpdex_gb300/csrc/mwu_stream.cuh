@@ -186,22 +186,26 @@ __device__ __forceinline__ bool pair_count(const PairTable& t, K key, uint32_t g
     return false;
 }
 
-// Whether a column's values repeat: of kTieSample entries, evenly spaced over it, more than one in
-// eight equal an earlier one. Sets bit 2 of flags[c] for the columns of at least 2 * kTieSample entries, one
-// block each, and bit 3 where more than five in eight do; repeat[c] is the share of the sample's pairs
-// that are equal (an estimate of the sum of squared frequencies of the column's values; 0 for the
-// columns not sampled). The plan decides by both (StreamRule).
+// How a column's values repeat, from kTieSample entries evenly spaced over it: `equal` of them equal an
+// earlier one, and `repeat` is the share of their pairs that are equal (an estimate of the sum of
+// squared frequencies of the column's values). Both 0 for columns of fewer than 2 * kTieSample entries; one
+// block a column. The plan decides by both (StreamRule).
+struct ColumnTies {
+    float repeat;
+    uint32_t equal;
+};
 constexpr int kTieSample = 512;
 template <class V>
-__global__ void __launch_bounds__(128) column_ties_kernel(const V* data, const int64_t* indptr, uint32_t* flags,
-                                                          float* repeat) {
+__global__ void __launch_bounds__(128) column_ties_kernel(const V* data, const int64_t* indptr, ColumnTies* ties) {
     using K = typename Val<V>::Key;
     __shared__ unsigned long long slot[2 * kTieSample];  // key + 1 (0: empty)
     __shared__ uint32_t more[2 * kTieSample];            // elements of the slot's value after its first
     __shared__ uint32_t equal, pairs, used;
     const long long b = indptr[blockIdx.x], n = indptr[blockIdx.x + 1] - b;
-    if (threadIdx.x == 0) repeat[blockIdx.x] = 0.0f;
-    if (n < 2 * kTieSample) return;
+    if (n < 2 * kTieSample) {
+        if (threadIdx.x == 0) ties[blockIdx.x] = ColumnTies{0.0f, 0u};
+        return;
+    }
     for (int i = threadIdx.x; i < 2 * kTieSample; i += 128) { slot[i] = 0ull; more[i] = 0u; }
     if (threadIdx.x == 0) { equal = 0u; pairs = 0u; used = 0u; }
     __syncthreads();
@@ -222,10 +226,8 @@ __global__ void __launch_bounds__(128) column_ties_kernel(const V* data, const i
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        if (equal > kTieSample / 8) flags[blockIdx.x] |= equal > 5 * kTieSample / 8 ? 12u : 4u;
-        if (used > 1u) repeat[blockIdx.x] = 2.0f * (float)pairs / ((float)used * (float)(used - 1u));
-    }
+    if (threadIdx.x == 0)
+        ties[blockIdx.x] = ColumnTies{used > 1u ? 2.0f * (float)pairs / ((float)used * (float)(used - 1u)) : 0.0f, equal};
 }
 
 // One 1,024-thread CTA per SM takes genes from the work queue. Per gene:
