@@ -1529,6 +1529,58 @@ int plan_create(hpdex_matrix* m, const int32_t* group_id, int64_t n_targets,
 
 }  // namespace
 
+namespace {
+// Sorts, adjusts and restores the order of n p-values, n >= 2 (fdr.cuh).
+template <int ITEMS>
+int bh_fdr(const double* p, int64_t n, double* fdr) {
+    DeviceInfo dev;
+    TRY(device_info(dev));
+    const int tile = kSortThreads * ITEMS, nb = (int)((n + tile - 1) / tile);
+    DevBuf<unsigned long long> k0, k1;
+    DevBuf<uint32_t> v0, v1, counts, totals, bad;
+    DevBuf<double> agg, carry, out;
+    TRY(k0.alloc((size_t)n));
+    TRY(k1.alloc((size_t)n));
+    TRY(v0.alloc((size_t)n));
+    TRY(v1.alloc((size_t)n));
+    TRY(counts.alloc((size_t)256 * nb));
+    TRY(totals.alloc(256));
+    TRY(bad.alloc(1));
+    TRY(agg.alloc((size_t)nb));
+    TRY(carry.alloc((size_t)nb));
+    TRY(out.alloc((size_t)n));
+    cudaStream_t s = 0;
+    CUDA_TRY(cudaMemcpyAsync(k0.p, p, sizeof(double) * n, cudaMemcpyHostToDevice, s));
+    CUDA_TRY(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), s));
+    if (kSortScatterSmem<ITEMS> > 48 * 1024) CUDA_TRY(allow_max_smem(radix_scatter_kernel<ITEMS>));
+    unsigned long long* kin = k0.p;
+    unsigned long long* kout = k1.p;
+    uint32_t* vin = nullptr;
+    uint32_t* vout = v1.p;
+    for (int pass = 0; pass < 8; ++pass) {
+        const int shift = 8 * pass;
+        radix_count_kernel<ITEMS><<<nb, kSortThreads, 0, s>>>(kin, n, shift, counts.p, nb);
+        radix_scan_kernel<<<256, kSortThreads, 0, s>>>(counts.p, nb, totals.p);
+        radix_scatter_kernel<ITEMS><<<nb, kSortThreads, kSortScatterSmem<ITEMS>, s>>>(kin, vin, kout, vout, n, shift, counts.p, totals.p, nb);
+        CUDA_TRY(cudaGetLastError());
+        std::swap(kin, kout);
+        vin = vout;
+        vout = (vout == v1.p) ? v0.p : v1.p;
+    }
+    double* adj = reinterpret_cast<double*>(kout);  // the sort's other key buffer is free now
+    bh_block_min_kernel<ITEMS><<<nb, kSortThreads, 0, s>>>(kin, n, adj, agg.p, bad.p);
+    bh_carry_kernel<<<1, 1024, 0, s>>>(agg.p, nb, carry.p);
+    bh_apply_kernel<ITEMS><<<nb, kSortThreads, 0, s>>>(adj, vin, n, carry.p, out.p);
+    CUDA_TRY(cudaGetLastError());
+    uint32_t bad_h = 0;
+    CUDA_TRY(cudaMemcpyAsync(&bad_h, bad.p, sizeof bad_h, cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    if (bad_h) return fail(HPDEX_ERR_ARGUMENT, "All values in `ps` must lie between 0. and 1.");
+    CUDA_TRY(cudaMemcpy(fdr, out.p, sizeof(double) * n, cudaMemcpyDeviceToHost));
+    return HPDEX_OK;
+}
+}  // namespace
+
 // =======================================================================================
 extern "C" {
 
@@ -1609,51 +1661,7 @@ int hpdex_bh_fdr(const double* p, int64_t n, double* fdr) {
         return HPDEX_OK;
     }
     if (n >= (1ll << 31)) return fail(HPDEX_ERR_UNSUPPORTED, "at most 2^31 - 1 p-values");
-    DeviceInfo dev;
-    TRY(device_info(dev));
-    const int nb = (int)((n + kSortTile - 1) / kSortTile);
-    DevBuf<unsigned long long> k0, k1;
-    DevBuf<uint32_t> v0, v1, counts, totals, bad;
-    DevBuf<double> agg, carry, out;
-    TRY(k0.alloc((size_t)n));
-    TRY(k1.alloc((size_t)n));
-    TRY(v0.alloc((size_t)n));
-    TRY(v1.alloc((size_t)n));
-    TRY(counts.alloc((size_t)256 * nb));
-    TRY(totals.alloc(256));
-    TRY(bad.alloc(1));
-    TRY(agg.alloc((size_t)nb));
-    TRY(carry.alloc((size_t)nb));
-    TRY(out.alloc((size_t)n));
-    cudaStream_t s = 0;
-    CUDA_TRY(cudaMemcpyAsync(k0.p, p, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    CUDA_TRY(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), s));
-    CUDA_TRY(allow_max_smem(radix_scatter_kernel));
-    unsigned long long* kin = k0.p;
-    unsigned long long* kout = k1.p;
-    uint32_t* vin = nullptr;
-    uint32_t* vout = v1.p;
-    for (int pass = 0; pass < 8; ++pass) {
-        const int shift = 8 * pass;
-        radix_count_kernel<<<nb, kSortThreads, 0, s>>>(kin, n, shift, counts.p, nb);
-        radix_scan_kernel<<<256, kSortThreads, 0, s>>>(counts.p, nb, totals.p);
-        radix_scatter_kernel<<<nb, kSortThreads, kSortScatterSmem, s>>>(kin, vin, kout, vout, n, shift, counts.p, totals.p, nb);
-        CUDA_TRY(cudaGetLastError());
-        std::swap(kin, kout);
-        vin = vout;
-        vout = (vout == v1.p) ? v0.p : v1.p;
-    }
-    double* adj = reinterpret_cast<double*>(kout);  // the sort's other key buffer is free now
-    bh_block_min_kernel<<<nb, kSortThreads, 0, s>>>(kin, n, adj, agg.p, bad.p);
-    bh_carry_kernel<<<1, 1024, 0, s>>>(agg.p, nb, carry.p);
-    bh_apply_kernel<<<nb, kSortThreads, 0, s>>>(adj, vin, n, carry.p, out.p);
-    CUDA_TRY(cudaGetLastError());
-    uint32_t bad_h = 0;
-    CUDA_TRY(cudaMemcpyAsync(&bad_h, bad.p, sizeof bad_h, cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaStreamSynchronize(s));
-    if (bad_h) return fail(HPDEX_ERR_ARGUMENT, "All values in `ps` must lie between 0. and 1.");
-    CUDA_TRY(cudaMemcpy(fdr, out.p, sizeof(double) * n, cudaMemcpyDeviceToHost));
-    return HPDEX_OK;
+    return n <= kSortSmall ? bh_fdr<4>(p, n, fdr) : bh_fdr<16>(p, n, fdr);
 }
 
 int hpdex_fold_change(const double* means, int64_t n_genes, int64_t n_groups, double clip,

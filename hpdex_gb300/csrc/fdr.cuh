@@ -10,7 +10,7 @@
 //
 // The sort is a stable LSD radix sort of the p-values' bit patterns (non-negative doubles
 // order like their bits) with 32-bit indices: 8 passes of 8-bit digits, each a count kernel
-// (digit counts of every tile of 4,096 entries), a scan kernel (one block per digit: prefix over
+// (digit counts of every tile of entries), a scan kernel (one block per digit: prefix over
 // the tiles) and a scatter kernel (per-warp stable ranks from warp match, the tile put in digit
 // order in shared memory, then written as runs). At 4 million p-values everything stays in L2
 // and a pass is bound by instruction issue. Per pass, before and after the tiles grew from 2,048
@@ -24,9 +24,12 @@
 namespace hpdex {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;                            // per thread and tile
-constexpr int kSortTile = kSortThreads * kSortItems;      // 4096 entries per block
 constexpr int kSortWarps = kSortThreads / 32;
+// ITEMS entries per thread: tiles of 4,096 entries (16) for many p-values, of 1,024 (4) up to
+// kSortSmall, where a pass is the time of one tile. A call with tiles of 1,024 / 2,048 / 4,096: 5,000
+// p-values 163 / 183 / 224 us, 60,000 175 / 209 / 253, 500,000 262 / 274 / 294, 1,500,000 483 / 464 / 492, 4,000,000
+// 1,023 / 977 / 970.
+constexpr long long kSortSmall = 1ll << 19;
 
 // -0.0 would sort after every positive value by its bits: it reads as +0.0 (they compare equal).
 __device__ __forceinline__ unsigned long long sort_key(unsigned long long k) {
@@ -34,15 +37,16 @@ __device__ __forceinline__ unsigned long long sort_key(unsigned long long k) {
 }
 
 // counts[d * ntiles + t]: entries of tile t with digit d.
+template <int ITEMS>
 __global__ void __launch_bounds__(kSortThreads) radix_count_kernel(const unsigned long long* keys,
                                                                    long long n, int shift,
                                                                    uint32_t* counts, int ntiles) {
     __shared__ uint32_t hist[256];
     hist[threadIdx.x] = 0u;
     __syncthreads();
-    const long long t0 = (long long)blockIdx.x * kSortTile;
+    const long long t0 = (long long)blockIdx.x * (kSortThreads * ITEMS);
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
+    for (int k = 0; k < ITEMS; ++k) {
         const long long i = t0 + (long long)k * kSortThreads + threadIdx.x;
         if (i < n) atomicAdd(&hist[(uint32_t)(sort_key(keys[i]) >> shift) & 255u], 1u);
     }
@@ -77,33 +81,35 @@ __global__ void __launch_bounds__(kSortThreads) radix_scan_kernel(uint32_t* coun
 }
 
 // Stable scatter of one pass. vin == nullptr: the values are the input positions. Dynamic shared
-// memory: kSortScatterSmem bytes.
-constexpr size_t kSortScatterSmem = (size_t)kSortTile * 12 + kSortWarps * 256 * 4;
+// memory: kSortScatterSmem<ITEMS> bytes.
+template <int ITEMS>
+constexpr size_t kSortScatterSmem = (size_t)kSortThreads * ITEMS * 12 + kSortWarps * 256 * 4;
+template <int ITEMS>
 __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
     const unsigned long long* kin, const uint32_t* vin, unsigned long long* kout, uint32_t* vout,
     long long n, int shift, const uint32_t* offsets, const uint32_t* totals, int ntiles) {
     extern __shared__ __align__(16) unsigned char sort_smem[];
     unsigned long long* skey = reinterpret_cast<unsigned long long*>(sort_smem);
-    uint32_t* sval = reinterpret_cast<uint32_t*>(skey + kSortTile);
-    uint32_t(*whist)[256] = reinterpret_cast<uint32_t(*)[256]>(sval + kSortTile);
+    uint32_t* sval = reinterpret_cast<uint32_t*>(skey + (kSortThreads * ITEMS));
+    uint32_t(*whist)[256] = reinterpret_cast<uint32_t(*)[256]>(sval + (kSortThreads * ITEMS));
     __shared__ uint32_t gofs[256];  // where the tile's first entry of a digit goes, minus its place
                                     // in the tile's digit order
     __shared__ uint32_t ws[2][kSortWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int d = threadIdx.x; d < kSortWarps * 256; d += kSortThreads) (&whist[0][0])[d] = 0u;
     __syncthreads();
-    // warp w takes the tile's entries [w*512, (w+1)*512), 32 consecutive ones per round
-    const long long base = (long long)blockIdx.x * kSortTile + (long long)warp * 32 * kSortItems;
-    unsigned long long key[kSortItems];
-    uint32_t place[kSortItems];  // digit << 16 | rank among the warp's entries of the digit
+    // warp w takes the tile's w-th part of 32 * ITEMS entries, 32 consecutive ones per round
+    const long long base = (long long)blockIdx.x * (kSortThreads * ITEMS) + (long long)warp * 32 * ITEMS;
+    unsigned long long key[ITEMS];
+    uint32_t place[ITEMS];  // digit << 16 | rank among the warp's entries of the digit
     const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const long long i = base + r * 32 + lane;
         key[r] = i < n ? sort_key(kin[i]) : 0ull;
     }
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const bool ok = base + r * 32 + lane < n;
         const uint32_t dig = ok ? ((uint32_t)(key[r] >> shift) & 255u) : 256u;
         const unsigned peers = __match_any_sync(0xffffffffu, dig);
@@ -133,7 +139,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const long long i = base + r * 32 + lane;
         if (i < n) {
             const uint32_t pos = whist[warp][place[r] >> 16] + (place[r] & 0xffffu);
@@ -142,7 +148,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
         }
     }
     __syncthreads();
-    const int cnt = (int)min((long long)kSortTile, n - (long long)blockIdx.x * kSortTile);
+    const int cnt = (int)min((long long)(kSortThreads * ITEMS), n - (long long)blockIdx.x * (kSortThreads * ITEMS));
 #pragma unroll 4
     for (int j = threadIdx.x; j < cnt; j += kSortThreads) {
         const unsigned long long k = skey[j];
@@ -160,14 +166,15 @@ __device__ __forceinline__ double bh_adjusted(const unsigned long long* sk, long
 
 // They are kept in adj (the division takes the narrow FP64 pipe: at 4 million values computing
 // them in both this kernel and bh_apply_kernel took 107 + 119 us, once 81 + 52 us).
+template <int ITEMS>
 __global__ void __launch_bounds__(kSortThreads) bh_block_min_kernel(const unsigned long long* sk,
                                                                      long long m, double* adj,
                                                                      double* agg, uint32_t* bad) {
     __shared__ unsigned long long ws[kSortWarps];
-    const long long t0 = (long long)blockIdx.x * kSortTile;
+    const long long t0 = (long long)blockIdx.x * (kSortThreads * ITEMS);
     unsigned long long v = 0x7ff0000000000000ull;  // +inf; non-negative doubles order like their bits
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
+    for (int k = 0; k < ITEMS; ++k) {
         const long long i = t0 + (long long)k * kSortThreads + threadIdx.x;
         if (i < m) {
             if (sk[i] > 0x3ff0000000000000ull) atomicOr(bad, 1u);  // NaN, negative or above 1
@@ -226,27 +233,28 @@ __global__ void __launch_bounds__(1024) bh_carry_kernel(const double* agg, int n
 
 // BH, step 3: suffix minimum inside each block plus its carry, clip, back to input order. The
 // tile goes through shared memory, so that global accesses are by neighbouring threads while a
-// thread scans 16 neighbouring values (one pad word per 16 keeps the banks apart); the values
+// thread scans ITEMS neighbouring values (one pad word after each keeps the banks apart); the values
 // are compared as integers (non-negative doubles), which leaves the narrow FP64 pipe out.
+template <int ITEMS>
 __global__ void __launch_bounds__(kSortThreads) bh_apply_kernel(const double* adj,
                                                                  const uint32_t* sv, long long m,
                                                                  const double* carry, double* fdr) {
     using U = unsigned long long;
-    __shared__ U tile[kSortTile + kSortThreads];
+    __shared__ U tile[kSortThreads * (ITEMS + 1)];
     __shared__ U ws[kSortWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long t0 = (long long)blockIdx.x * kSortTile;
+    const long long t0 = (long long)blockIdx.x * (kSortThreads * ITEMS);
     const U inf = 0x7ff0000000000000ull;
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
+    for (int k = 0; k < ITEMS; ++k) {
         const int j = k * kSortThreads + (int)threadIdx.x;
-        tile[j + j / kSortItems] = t0 + j < m ? (U)__double_as_longlong(adj[t0 + j]) : inf;
+        tile[j + j / ITEMS] = t0 + j < m ? (U)__double_as_longlong(adj[t0 + j]) : inf;
     }
     __syncthreads();
-    U* mine = tile + (int)threadIdx.x * (kSortItems + 1);
+    U* mine = tile + (int)threadIdx.x * (ITEMS + 1);
     U tmin = inf;
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) tmin = min(tmin, mine[k]);
+    for (int k = 0; k < ITEMS; ++k) tmin = min(tmin, mine[k]);
     // min over the threads after this one (tile order = thread order)
     U incl = tmin;
     for (int o = 1; o < 32; o <<= 1) {
@@ -260,15 +268,15 @@ __global__ void __launch_bounds__(kSortThreads) bh_apply_kernel(const double* ad
     for (int w = warp + 1; w < kSortWarps; ++w) after = min(after, ws[w]);
     after = min(after, (U)__double_as_longlong(carry[blockIdx.x]));
 #pragma unroll
-    for (int k = kSortItems - 1; k >= 0; --k) {
+    for (int k = ITEMS - 1; k >= 0; --k) {
         after = min(after, mine[k]);
         mine[k] = min(after, (U)0x3ff0000000000000ull);  // at most 1
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
+    for (int k = 0; k < ITEMS; ++k) {
         const int j = k * kSortThreads + (int)threadIdx.x;
-        if (t0 + j < m) fdr[sv[t0 + j]] = __longlong_as_double((long long)tile[j + j / kSortItems]);
+        if (t0 + j < m) fdr[sv[t0 + j]] = __longlong_as_double((long long)tile[j + j / ITEMS]);
     }
 }
 
