@@ -2770,22 +2770,47 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
     }
     std::vector<int32_t> order[3];
     std::vector<uint16_t> order_task[3];
-    auto put = [&](int list, int32_t c, size_t i) {
-        order[list].push_back(c);
-        order_task[list].push_back((uint16_t)i);
-    };
     long long taken = 0, rest_ints = 0, rest_floats = 0;  // entries
+    // the list of all genes of a query, where they share one: whole classes are appended then (8,000
+    // genes one by one took 25 us of a query's 700)
+    std::vector<int> common(b.q.size(), -1);
+    size_t room[3] = {0, 0, 0};
+    for (size_t i = 0; i < b.q.size(); ++i) {
+        const hpdex_matrix* m = S->mats[(size_t)b.q[i]->matrix];
+        if (stream[i] || (hist_smem && m->n_int_cols > 0 && m->n_int_cols < m->n_cols)) {
+            for (size_t& r : room) r += (size_t)m->n_cols;
+            continue;
+        }
+        common[i] = hist_smem && m->n_int_cols > 0 ? 0 : 2;
+        room[common[i]] += (size_t)m->n_cols;
+        if (common[i] == 0) {
+            taken += m->int_entries;
+        } else {
+            rest_ints += m->int_entries;
+            rest_floats += m->nnz - m->int_entries;
+        }
+    }
+    for (int l = 0; l < 3; ++l) {
+        order[l].reserve(room[l]);
+        order_task[l].reserve(room[l]);
+    }
     for (int k = 63; k >= 0; --k)
         for (size_t i = 0; i < b.q.size(); ++i) {
             const hpdex_matrix* m = S->mats[(size_t)b.q[i]->matrix];
             const auto& ord = S->mat_order[(size_t)b.q[i]->matrix];
             const auto& seg = S->mat_class_start[(size_t)b.q[i]->matrix];
             const int64_t lo = seg[(size_t)(2 * k)], hi = seg[(size_t)(2 * k + 1)];
+            if (common[i] >= 0) {
+                order[common[i]].insert(order[common[i]].end(), ord.begin() + lo, ord.begin() + hi);
+                order_task[common[i]].insert(order_task[common[i]].end(), (size_t)(hi - lo), (uint16_t)i);
+                continue;
+            }
             for (int64_t j = lo; j < hi; ++j) {
                 const int32_t c = ord[(size_t)j];
                 const bool is_int = m->int_col((size_t)c);
                 const int list = hist_smem && is_int ? 0 : stream[i] && stream[i]->takes((size_t)c) ? 1 : 2;
-                put(list, c, i);
+                order[list].push_back(c);
+                order_task[list].push_back((uint16_t)i);
                 if (list != 1) (list == 0 ? taken : is_int ? rest_ints : rest_floats) += m->col_nnz[(size_t)c];
             }
         }
