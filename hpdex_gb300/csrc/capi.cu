@@ -957,7 +957,8 @@ long long stream_longest(const DeviceInfo& dev, int dtype, int G, long long ref_
 // 1.5 (110) 0.87.
 // Short genes, whose buckets and barriers cost more here, most so for doubles: at 1,100 / 2,000 / 3,000 / 7,000
 // entries float32 log values 0.94 / 0.97 / 1.17 / 1.27 (90 targets), double 0.77 / 0.82 / 0.98 / 1.11, and 0.87 /
-// 0.88 / 1.01 / 0.97 at 300 targets, 1.20 at 15,000.
+// 0.88 / 1.01 / 0.97 at 300 targets, 1.20 at 15,000; float32 at 4 targets 1.03 / 1.19 / 1.37 / 1.71, and 0.91 at 1,500
+// where 1,800 values repeat.
 constexpr double kStreamRepeats = 0.6;
 struct StreamRule {
     const hpdex_matrix* m;
@@ -985,9 +986,9 @@ struct StreamRule {
     }
     // a gene of fewer entries is not counted for the stream kernel (kStreamAny: not taken either)
     long long least(size_t c) const {
-        const bool repeats = m->col_repeat[c] > 1.0f / 20000.0f;
+        const bool repeats = m->col_repeat[c] > 1.0f / 5000.0f;
         if (m->dtype == HPDEX_FLOAT64) return n_targets > 100 ? 12000 : repeats ? 6000 : n_targets > 20 ? 4500 : 3000;
-        return level == kStreamGroups ? kStreamMinEntries : repeats || n_targets > 20 ? 2500 : 1500;
+        return level == kStreamGroups ? kStreamMinEntries : repeats || n_targets > 60 ? 2500 : n_targets > 10 ? 2000 : 1500;
     }
     bool takes(size_t c) const {
         const long long n = m->col_nnz[c];

@@ -22,7 +22,8 @@ CASES = [
     (np.float32, 170_000, 20_000, 60, 0.0, False),  # 0.13, but little room beside the reference
     (np.float32, 1_300, 0, 5, 0.0, False),
     (np.float32, 2_000, 0, 5, 0.0, True),
-    (np.float32, 2_000, 0, 50, 0.0, False),
+    (np.float32, 2_200, 0, 50, 0.0, True),
+    (np.float32, 2_200, 0, 80, 0.0, False),
     (np.float64, 2_800, 0, 5, 0.0, False),
     (np.float64, 4_000, 0, 5, 0.0, True),
     (np.float64, 4_000, 0, 50, 0.0, False),
