@@ -968,6 +968,8 @@ struct StreamRule {
     long long n_targets, longest;
     double room;                                    // bytes for reference, bitmaps and table
     double key;
+    std::vector<uint8_t> taken;                     // per gene, once pays() is asked
+    bool all = false;                               // every one
 
     StreamRule(const hpdex_matrix* matrix, const std::vector<long long>& group_rows, int layout_g, bool tie_correction,
                uint8_t stream_level)
@@ -997,25 +999,33 @@ struct StreamRule {
     double repeats(size_t c) const {
         if (!ties) return 0.0;  // (no second pass)
         const double n = (double)m->col_nnz[c], t = n * targets, p = (double)m->col_repeat[c];
+        const double pairs = t * p / spread;
+        if (n * p <= 4.0) return pairs;
         const double space = std::max(room - n * ref * (key + 2.0), 1024.0);
         const double cells = 8.0 * std::min(space / 2.0, std::max(8.0 * t, t * t / 4.0) + 16.0);
-        return t * p / spread + (n * p > 4.0 ? 2.0 * t / cells : 0.0);
+        return pairs + 2.0 * t / cells;
     }
-    bool pays() const {
+    bool pays() {
         if (m->col_stream.empty() || longest <= 0) return false;
-        long long all = 0, held = 0, rest_longest = 0;  // (held: entries of the genes long enough)
-        double taken = 0.0, work = 0.0;
-        for (size_t c = 0; c < m->col_nnz.size(); ++c) {
+        const size_t C = m->col_nnz.size();
+        long long entries = 0, held = 0, rest_longest = 0;  // (held: entries of the genes long enough)
+        double weight = 0.0, work = 0.0;
+        size_t count = 0;
+        taken.assign(C, 0);
+        for (size_t c = 0; c < C; ++c) {
             const long long n = m->col_nnz[c];
             if (m->int_col(c)) continue;
-            all += n;
+            entries += n;
             if (!takes(c)) { rest_longest = std::max(rest_longest, n); continue; }
-            if (n >= least(c)) held += n;
-            taken += (double)n;
+            taken[c] = 1;
+            ++count;
+            if (level == kStreamAny || n >= least(c)) held += n;
+            weight += (double)n;
             work += (double)n * repeats(c);
         }
-        return held > 0 && held * 100 >= all * kStreamMinPercent && work <= kStreamRepeats * taken &&
-               (level == kStreamAny || rest_longest * kStreamRestShare * m->dev.sms <= all);
+        all = count == C;
+        return held > 0 && held * 100 >= entries * kStreamMinPercent && work <= kStreamRepeats * weight &&
+               (level == kStreamAny || rest_longest * kStreamRestShare * m->dev.sms <= entries);
     }
 };
 
@@ -1090,7 +1100,7 @@ int divide_genes(hpdex_plan* p, const RankLayout& r) {
         if (p->hist_smem && m->int_col((size_t)c)) {
             hist.push_back(c);
             taken += n;
-        } else if (all_stream || (rule && rule->takes((size_t)c))) {
+        } else if (all_stream || (rule && rule->taken[(size_t)c])) {
             stream.push_back(c);
         } else {
             rest.push_back(c);
@@ -2778,15 +2788,16 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
     size_t room[3] = {0, 0, 0};
     for (size_t i = 0; i < b.q.size(); ++i) {
         const hpdex_matrix* m = S->mats[(size_t)b.q[i]->matrix];
-        if (stream[i] || (hist_smem && m->n_int_cols > 0 && m->n_int_cols < m->n_cols)) {
+        const bool ints = hist_smem && m->n_int_cols > 0;
+        if (stream[i] ? !stream[i]->all : ints && m->n_int_cols < m->n_cols) {
             for (size_t& r : room) r += (size_t)m->n_cols;
             continue;
         }
-        common[i] = hist_smem && m->n_int_cols > 0 ? 0 : 2;
+        common[i] = stream[i] ? 1 : ints ? 0 : 2;
         room[common[i]] += (size_t)m->n_cols;
         if (common[i] == 0) {
             taken += m->int_entries;
-        } else {
+        } else if (common[i] == 2) {
             rest_ints += m->int_entries;
             rest_floats += m->nnz - m->int_entries;
         }
@@ -2809,7 +2820,7 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
             for (int64_t j = lo; j < hi; ++j) {
                 const int32_t c = ord[(size_t)j];
                 const bool is_int = m->int_col((size_t)c);
-                const int list = hist_smem && is_int ? 0 : stream[i] && stream[i]->takes((size_t)c) ? 1 : 2;
+                const int list = hist_smem && is_int ? 0 : stream[i] && stream[i]->taken[(size_t)c] ? 1 : 2;
                 order[list].push_back(c);
                 order_task[list].push_back((uint16_t)i);
                 if (list != 1) (list == 0 ? taken : is_int ? rest_ints : rest_floats) += m->col_nnz[(size_t)c];
