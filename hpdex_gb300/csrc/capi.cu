@@ -419,8 +419,21 @@ struct hpdex_matrix {
     DevBuf<unsigned char> data;
     DevBuf<int32_t> rows;
     DevBuf<int64_t> indptr;
-    DevBuf<unsigned long long> col_kmin, col_kmax;  // per-column key range (resident layout)
-    DevBuf<uint32_t> col_has_zero;
+    // per-column key range and flags (resident layout), one after the other in one block, which the
+    // host fetches in one copy
+    template <class T>
+    struct Part { T* p = nullptr; };
+    DevBuf<unsigned long long> col_stats;
+    Part<unsigned long long> col_kmin, col_kmax;
+    Part<uint32_t> col_has_zero;
+    int alloc_col_stats(long long cols) {
+        const size_t c = (size_t)std::max<long long>(cols, 1);
+        TRY(col_stats.alloc(2 * c + (c + 1) / 2));
+        col_kmin.p = col_stats.p;
+        col_kmax.p = col_stats.p + c;
+        col_has_zero.p = reinterpret_cast<uint32_t*>(col_stats.p + 2 * c);
+        return HPDEX_OK;
+    }
     std::vector<long long> col_nnz;  // host copy for scheduling
     long long max_col_nnz = 0;
     // resident float matrices: which columns may take the stream kernel (kStreamAny, kStreamGroups;
@@ -647,11 +660,10 @@ int matrix_int_hint(hpdex_matrix* m) {
     m->has_int_cols = false;
     if (C == 0) return HPDEX_OK;
     const bool floats = m->dtype == HPDEX_FLOAT32 || m->dtype == HPDEX_FLOAT64;
-    std::vector<uint32_t> f((size_t)C);
-    std::vector<unsigned long long> lo((size_t)C), hi((size_t)C);
-    CUDA_TRY(cudaMemcpy(f.data(), m->col_has_zero.p, sizeof(uint32_t) * C, cudaMemcpyDeviceToHost));
-    CUDA_TRY(cudaMemcpy(lo.data(), m->col_kmin.p, sizeof(unsigned long long) * C, cudaMemcpyDeviceToHost));
-    CUDA_TRY(cudaMemcpy(hi.data(), m->col_kmax.p, sizeof(unsigned long long) * C, cudaMemcpyDeviceToHost));
+    std::vector<unsigned long long> stats(m->col_stats.n);
+    CUDA_TRY(cudaMemcpy(stats.data(), m->col_stats.p, sizeof(unsigned long long) * stats.size(), cudaMemcpyDeviceToHost));
+    const unsigned long long *lo = stats.data(), *hi = lo + C;
+    const uint32_t* f = reinterpret_cast<const uint32_t*>(hi + C);
     auto empty = [&](size_t c) { return lo[c] > hi[c]; };
     auto small_ints = [&](size_t c) { return !(f[c] & 2u) && !empty(c); };
     long long ints = 0, others = 0;
@@ -662,7 +674,7 @@ int matrix_int_hint(hpdex_matrix* m) {
         m->col_int.resize((size_t)C);
         for (long long c = 0; c < C; ++c) m->col_int[(size_t)c] = empty((size_t)c) ? ints > others : small_ints((size_t)c);
     }
-    if (floats && others > 0) {
+    if (floats && others > 0 && m->max_col_nnz >= 2 * kTieSample) {  // (else no column is sampled)
         DevBuf<ColumnTies> d_ties;
         std::vector<ColumnTies> ties((size_t)C);
         TRY(d_ties.alloc((size_t)C));
@@ -768,9 +780,7 @@ int upload_matrix(hpdex_matrix* m, const void* data, const int64_t* indices, con
         CUDA_TRY(cudaDeviceSynchronize());
     }
     // per-column key range of finite nonzero values: the bucket function of every plan
-    TRY(m->col_kmin.alloc(std::max<long long>(m->n_cols, 1)));
-    TRY(m->col_kmax.alloc(std::max<long long>(m->n_cols, 1)));
-    TRY(m->col_has_zero.alloc(std::max<long long>(m->n_cols, 1)));
+    TRY(m->alloc_col_stats(m->n_cols));
     if (m->n_cols) {
         TRY(dispatch_dtype<KeyRangeLaunch>(m->dtype, (const void*)m->data.p, (const int64_t*)m->indptr.p, m->n_cols,
                                            m->col_kmin.p, m->col_kmax.p, m->col_has_zero.p, m->nnz, m->dev.sms,
@@ -990,7 +1000,7 @@ struct StreamRule {
     long long least(size_t c) const {
         const bool repeats = m->col_repeat[c] > 1.0f / 5000.0f;
         if (m->dtype == HPDEX_FLOAT64) return n_targets > 100 ? 12000 : repeats ? 6000 : n_targets > 20 ? 4500 : 3000;
-        return level == kStreamGroups ? kStreamMinEntries : repeats || n_targets > 60 ? 2500 : n_targets > 10 ? 2000 : 1500;
+        return level == kStreamGroups ? kStreamMinEntries : repeats || n_targets > 60 ? 2500 : n_targets > 10 ? 1800 : 1500;
     }
     bool takes(size_t c) const {
         const long long n = m->col_nnz[c];
@@ -2167,9 +2177,7 @@ int matrix_create_csr(int32_t dtype, const void* data, const GI* indices, const 
     m->nnz = nnz;
     TRY(device_info(m->dev));
     TRY(dispatch_dtype<TransposeLaunch>(dtype, m.get(), data, indices, indptr));
-    TRY(m->col_kmin.alloc(std::max<long long>(n_cols, 1)));
-    TRY(m->col_kmax.alloc(std::max<long long>(n_cols, 1)));
-    TRY(m->col_has_zero.alloc(std::max<long long>(n_cols, 1)));
+    TRY(m->alloc_col_stats(n_cols));
     if (n_cols) {
         TRY(dispatch_dtype<KeyRangeLaunch>(dtype, (const void*)m->data.p, (const int64_t*)m->indptr.p, m->n_cols,
                                            m->col_kmin.p, m->col_kmax.p, m->col_has_zero.p, m->nnz, m->dev.sms,
@@ -2301,9 +2309,7 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
     TRY(m->data.alloc(std::max<size_t>(1, (size_t)nnz * vs)));
     TRY(m->rows.alloc(std::max<long long>(1, nnz)));
     TRY(m->indptr.alloc((size_t)C + 1));
-    TRY(m->col_kmin.alloc(std::max<long long>(C, 1)));
-    TRY(m->col_kmax.alloc(std::max<long long>(C, 1)));
-    TRY(m->col_has_zero.alloc(std::max<long long>(C, 1)));
+    TRY(m->alloc_col_stats(C));
     m->col_nnz.resize((size_t)C);
     for (long long c = 0; c < C; ++c) {
         m->col_nnz[(size_t)c] = indptr[c + 1] - indptr[c];
