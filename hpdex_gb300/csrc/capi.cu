@@ -71,26 +71,27 @@ constexpr int kPlainStreams = 128;  // concurrent streams of the plain form (the
 constexpr int kMeanThreads = 256;
 constexpr int kMeanFixedThreads = 512;
 
-// Whether a kernel may write the caller's doubles (`bytes` > 0) at `p` because they are page-locked: the first
-// and the last byte, so that an array registered in part is not written past its registration.
-bool page_locked(const void* p, size_t bytes) {
-    const unsigned char* ends[2] = {static_cast<const unsigned char*>(p), static_cast<const unsigned char*>(p) + bytes - 1};
-    bool ok = p != nullptr && bytes > 0 && reinterpret_cast<uintptr_t>(p) % sizeof(double) == 0;
-    for (int k = 0; k < 2 && ok; ++k) {
-        cudaPointerAttributes at{};
-        ok = cudaPointerGetAttributes(&at, ends[k]) == cudaSuccess && at.type == cudaMemoryTypeHost &&
-             at.devicePointer == ends[k];
-    }
-    cudaGetLastError();
-    return ok;
-}
-
 struct DeviceInfo {
     int device = -1;
     int sms = 0;
     size_t smem_per_sm = 0, smem_optin = 0, smem_reserved = 0;
     bool pageable_access = false;
 };
+
+// Whether a kernel may write the caller's doubles (`bytes` > 0) at `p` because they are page-locked. Where the
+// device does not reach pageable memory the last byte counts as well as the first, so that an array
+// registered in part is not written past its registration.
+bool page_locked(const DeviceInfo& dev, const void* p, size_t bytes) {
+    auto locked = [](const unsigned char* at) {
+        cudaPointerAttributes a{};
+        const bool ok = cudaPointerGetAttributes(&a, at) == cudaSuccess && a.type == cudaMemoryTypeHost && a.devicePointer == at;
+        cudaGetLastError();
+        return ok;
+    };
+    const unsigned char* b = static_cast<const unsigned char*>(p);
+    return p != nullptr && bytes > 0 && reinterpret_cast<uintptr_t>(p) % sizeof(double) == 0 && locked(b) &&
+           (dev.pageable_access || locked(b + bytes - 1));
+}
 
 // Properties of the current device, queried once per device and process.
 int device_info(DeviceInfo& d) {
@@ -2226,7 +2227,7 @@ int matrix_group_mean(const hpdex_matrix* m, const int32_t* group_id, int64_t n_
     TRY(grows.alloc(G));
     if (fixed) TRY(gid16.alloc(std::max<long long>(n_rows, 1)));
     // a page-locked result buffer is written by the kernel itself
-    const bool direct = page_locked(out, sizeof(double) * (size_t)n_cols * G);
+    const bool direct = page_locked(m->dev, out, sizeof(double) * (size_t)n_cols * G);
     if (!direct) TRY(dout.alloc((size_t)n_cols * G));
     const int grid = fixed ? (int)n_cols : (int)std::min<long long>(n_cols, (long long)m->dev.sms * 4);
     if (!fixed) TRY(acc.alloc((size_t)grid * 16 * G));
@@ -2468,7 +2469,7 @@ int oneshot_pipelined(int32_t dtype, const void* data, const int64_t* indices, c
     // Page-locked outputs (hpdex_host_buffer_acquire) are written directly on any system and
     // need no touching; pageable ones directly where the device can reach pageable memory.
     const size_t out_bytes = sizeof(double) * (size_t)(p->T * C);
-    const bool pinned_out = page_locked(U1_out, out_bytes) && page_locked(P_out, out_bytes);
+    const bool pinned_out = page_locked(m->dev, U1_out, out_bytes) && page_locked(m->dev, P_out, out_bytes);
     const bool direct = (m->dev.pageable_access || pinned_out) && U1_out && P_out;
     std::atomic<int> touched{pinned_out ? 1 : 0};
     struct Toucher {
@@ -2854,7 +2855,7 @@ int server_launch(hpdex_server* S, ServerBatch& b) {
     // that were never written would fault one by one when the device writes them: touch them
     for (ServerQuery* q : b.q) {
         const size_t bytes = sizeof(double) * (size_t)(q->T * S->mats[(size_t)q->matrix]->n_cols);
-        const bool pinned = page_locked(q->U1_out, bytes) && page_locked(q->P_out, bytes);
+        const bool pinned = page_locked(S->dev, q->U1_out, bytes) && page_locked(S->dev, q->P_out, bytes);
         q->direct = pinned || S->dev.pageable_access;
         if (!q->direct || pinned) continue;
         for (size_t o = 0; o < bytes; o += 4096) {
