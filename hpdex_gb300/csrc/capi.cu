@@ -1104,8 +1104,13 @@ int divide_genes(hpdex_plan* p, const RankLayout& r) {
     }
     const bool histogram = p->hist_on && m->has_int_cols;
     p->hist_smem = histogram && !all_stream ? hist_layout(m->dev, G, m->n_int_cols, m->int_longest, m->int_entries, r, &p->ha) : 0;
+    if (!all_stream && !rule && !(p->hist_smem && m->n_int_cols > 0)) {  // the rank kernel takes p->order
+        p->rest_histogram = histogram && with_histogram(m->int_entries, m->nnz - m->int_entries, 0);
+        return HPDEX_OK;
+    }
     std::vector<int32_t> hist, stream, rest;
     long long taken = 0, rest_ints = 0, rest_floats = 0;  // entries
+    for (auto* v : {&hist, &stream}) v->reserve(order.size());
     for (const int32_t c : order) {
         const long long n = m->col_nnz[(size_t)c];
         if (p->hist_smem && m->int_col((size_t)c)) {
@@ -1119,7 +1124,7 @@ int divide_genes(hpdex_plan* p, const RankLayout& r) {
         }
     }
     p->rest_histogram = histogram && with_histogram(rest_ints, rest_floats, taken);
-    if (hist.empty() && stream.empty()) return HPDEX_OK;  // the rank kernel takes p->order
+    if (hist.empty() && stream.empty()) return HPDEX_OK;
 
     auto upload = [&](DevBuf<int32_t>& d, const std::vector<int32_t>& genes) -> int {
         TRY(d.alloc(genes.size() == order.size() ? 0 : genes.size()));
