@@ -74,3 +74,22 @@ def test_integer_plans_of_different_group_counts():
                         np.testing.assert_array_equal(a, b)
         jobs.append(job)
     assert not _together(jobs)
+
+
+def test_csr_transposes_of_different_widths():
+    from hpdex_gb300.resident import ResidentMatrix
+    jobs = []
+    for cols in (200, 15_000, 38_000):  # counters of 800 bytes, 60 and 152 KB
+        rng = np.random.default_rng(cols)
+        rows, per = 300, 40
+        genes = np.concatenate([np.sort(rng.choice(cols, per, replace=False)) for _ in range(rows)]).astype(np.int64)
+        data = rng.integers(1, 9, genes.size).astype(np.float32)
+        want = np.bincount(genes, weights=data, minlength=cols) / rows
+
+        def job(cols=cols, genes=genes, data=data, want=want):
+            for _ in range(60):
+                m = ResidentMatrix.from_csr(data, genes, np.arange(rows + 1) * per, rows, cols)
+                np.testing.assert_array_equal(m.group_mean(np.zeros(rows, np.int32), 1), want)
+                m.close()
+        jobs.append(job)
+    assert not _together(jobs)
