@@ -645,8 +645,8 @@ struct MeanLaunch {  // smem 0: accumulators in global memory
 // matrix on each: 200 + 410 us, all on the rank kernel 430). Plans of more than kStreamManyGroups
 // groups, whose (value, group) pairs repeat less than the values do, take it up to five values
 // in eight repeating (kStreamGroups), and then for short genes as well. The gain is small there (the
-// log1p-CP10k screen of 500 targets 3.14 / 2.90 ms), so no gene behind it may be longer than 1/kStreamRestShare of what an SM gets (a few genes of 110,000
-// entries left of 1.8e7: 0.85 / 1.39 ms).
+// log1p-CP10k screen of 500 targets 3.14 / 2.90 ms), so no gene behind it may be longer than
+// 1/kStreamRestShare of what an SM gets (a few genes of 110,000 entries left of 1.8e7: 0.85 / 1.39 ms).
 constexpr long long kStreamMinEntries = 1024;
 constexpr long long kStreamMinPercent = 95;
 constexpr long long kStreamManyGroups = 100;

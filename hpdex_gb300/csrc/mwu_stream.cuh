@@ -15,16 +15,16 @@
 //     as it needs.
 // The work per entry is the same for 37 groups of 400 elements and 1,500 of 20, and none of it
 // depends on a slab of the gene fitting in shared memory, which holds the sorted reference, the
-// accumulators and the table. A gene whose reference does not fit, or whose reference values
-// crowd a bucket, is listed for mwu_rank_kernel, launched behind this one.
+// accumulators and the table. A gene whose reference does not fit, whose reference values
+// crowd a bucket or one of whose pairs occurs more than 65,535 times is listed for mwu_rank_kernel,
+// launched behind this one.
 //
 // It gains where values seldom repeat: there mwu_rank_kernel resolves every bucket of several
 // values pairwise (continuous data at 60,000 entries a gene: 5 times the time), while here only
 // the first pass over a gene is bound by memory and the rest by instruction issue. Where a few
 // values hold most elements its second pass costs more than the one-value buckets of
 // mwu_rank_kernel (1,000 genes of 10,000 entries and 20 groups, 100 steps of a normal: 0.31 against
-// 0.21 ms). column_ties_kernel and the plan
-// (stream_genes) divide the genes.
+// 0.21 ms). column_ties_kernel's sample and the plan's grouping (StreamRule) divide the genes.
 #pragma once
 #include "mwu_rank.cuh"
 
@@ -136,6 +136,7 @@ __device__ __forceinline__ uint32_t ors(uint32_t p, uint32_t v) {
 }
 
 // Hash of a (key, group) pair: the high bits choose the cell or slot, the low ones the partition.
+// (Multipliers of MurmurHash3's finaliser and of xxHash.)
 __device__ __forceinline__ uint32_t pair_hash(uint32_t key, uint32_t g) {
     uint32_t h = key * 0x85ebca6bu + g * 0x9e3779b1u;
     h ^= h >> 15;
